@@ -78,9 +78,9 @@ SIGNATURES = {
     "cubit_listing_assemble": (C.c_int, [C.c_void_p, C.c_char_p, C.c_char_p, C.c_void_p, C.c_uint64, u64p, u64p]),
     "cubit_patch_elf": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint64, u64p, C.POINTER(PatchStats)]),
     "cubit_elf_patch_text": (C.c_int, [C.c_void_p, C.c_uint32, C.c_void_p, C.c_uint64, C.c_void_p, C.c_uint64, u64p]),
-    "cubit_disassemble": (C.c_int, [C.c_void_p, C.c_void_p, C.c_char_p, C.c_int, C.c_char_p, C.c_uint64, u64p, u64p]),
+    "cubit_disassemble": (C.c_int, [C.c_void_p, C.c_void_p, C.c_char_p, C.c_int, C.c_void_p, C.c_uint64, u64p, u64p]),
     "cubit_text_print": (C.c_int, [C.c_void_p, C.c_void_p, C.c_uint64, C.c_uint32, C.c_void_p, C.c_void_p, C.c_void_p,
-                                   C.c_char_p, C.c_uint64, u64p]),
+                                   C.c_void_p, C.c_uint64, u64p]),
 }
 
 _lib = None

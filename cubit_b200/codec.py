@@ -307,42 +307,40 @@ class Codec:
         self._check(self._lib.cubit_text_parse(self._ctx, text, addr, buf, need.value, need))
         return json.loads(buf.value.decode())
 
+    @staticmethod
+    def _most_statements(raw: bytes, program: bool) -> int:
+        """Upper bound of the instructions in a text: statements end at line ends and semicolons."""
+        return raw.count(b"\n") + raw.count(b";") + 1 if program else 1
+
+    def _check_text(self, rc: int):
+        if rc == ERR_TEXT:
+            raise ValueError(self._lib.cubit_last_error(self._ctx).decode())
+        self._check(rc)
+
     def lower_text(self, text: str, addr: int = 0, program: bool = True):
         """Text -> (form, slots, ctrl, clear, set): the records cubit_encode_batch takes and the
         128-bit patches ((word & ~clear) | set) that carry the text-derived bits.  clear / set
         are uint8[n, 16] little-endian.  ValueError with the reference's message on failure."""
-        mode = TEXT_PROGRAM if program else TEXT_ONE
         raw = text.encode()
+        cap = self._most_statements(raw, program)
         n = C.c_uint64()
-        rc = self._lib.cubit_text_lower(self._ctx, raw, addr, mode, 0, None, None, None, None, None, n)
-        if rc == ERR_TEXT:
-            raise ValueError(self._lib.cubit_last_error(self._ctx).decode())
-        self._check(rc)
-        cap = max(int(n.value), 1)
-        form = np.zeros(cap, np.uint16); slots = np.zeros((8, cap), np.uint32); ctrl = np.zeros(cap, np.uint32)
-        clear = np.zeros((cap, 16), np.uint8); set_ = np.zeros((cap, 16), np.uint8)
-        self._check(self._lib.cubit_text_lower(self._ctx, raw, addr, mode, cap, _ptr(form), _ptr(slots), _ptr(ctrl),
-                                               _ptr(clear), _ptr(set_), n))
-        k = int(n.value)
-        return form[:k], slots[:, :k], ctrl[:k], clear[:k], set_[:k]
+        form = np.empty(cap, np.uint16); slots = np.empty((8, cap), np.uint32); ctrl = np.empty(cap, np.uint32)
+        clear = np.empty((cap, 16), np.uint8); set_ = np.empty((cap, 16), np.uint8)
+        self._check_text(self._lib.cubit_text_lower(self._ctx, raw, addr, TEXT_PROGRAM if program else TEXT_ONE, cap, _ptr(form),
+                                                    _ptr(slots), _ptr(ctrl), _ptr(clear), _ptr(set_), n))
+        k = n.value
+        return form[:k], np.ascontiguousarray(slots[:, :k]), ctrl[:k], clear[:k], set_[:k]
 
     def encode_text(self, text: str, addr: int = 0, program: bool = True) -> np.ndarray:
         """Text -> uint8[n, 16] words.  `program=False`: one bare instruction, as the reference's
         encode(sass, addr); `program=True`: statements with labels, comments and optional
         control-code prefixes, as its assembler reads them (without its scheduling pass)."""
-        mode = TEXT_PROGRAM if program else TEXT_ONE
         raw = text.encode()
         n = C.c_uint64()
-        rc = self._lib.cubit_text_encode(self._ctx, raw, addr, mode, 0, None, n)
-        if rc == ERR_TEXT:
-            raise ValueError(self._lib.cubit_last_error(self._ctx).decode())
-        self._check(rc)
-        words = np.zeros((max(int(n.value), 1), 16), np.uint8)
-        rc = self._lib.cubit_text_encode(self._ctx, raw, addr, mode, len(words), _ptr(words), n)
-        if rc == ERR_TEXT:
-            raise ValueError(self._lib.cubit_last_error(self._ctx).decode())
-        self._check(rc)
-        return words[:int(n.value)]
+        words = np.empty((self._most_statements(raw, program), 16), np.uint8)
+        self._check_text(self._lib.cubit_text_encode(self._ctx, raw, addr, TEXT_PROGRAM if program else TEXT_ONE, len(words),
+                                                     _ptr(words), n))
+        return words[:n.value]
 
     def print_text(self, words, addr: int = 0, records=None) -> list[str]:
         """SASS text of each 16-byte word (uint8[n, 16]); word i is taken to sit at addr + 16 i.
@@ -361,13 +359,13 @@ class Codec:
         need = C.c_uint64()
         cap = 96 * n + 64                      # nearly always enough; the call reports the exact size otherwise
         for _ in range(2):
-            buf = C.create_string_buffer(cap)
+            buf = np.empty(cap, np.uint8)
             self._check(self._lib.cubit_text_print(self._ctx, _ptr(words), n, addr, _ptr(form), _ptr(slots), _ptr(ctrl),
-                                                   buf, cap, need))
+                                                   _ptr(buf), cap, need))
             if need.value <= cap:
                 break
             cap = need.value
-        return buf.value.decode().split("\n")[:n]
+        return str(buf[:need.value - 1].data, "utf-8").split("\n")[:n]
 
     def to_sass(self, lo: int, hi: int, addr: int = 0) -> str:
         """cubit.to_sass(lo, hi, addr=0) (reference src/python.rs:186-197)."""
@@ -478,14 +476,14 @@ class Codec:
                 total += size.value // 16
             cap = 112 * total + 512 * n_text + 64   # nearly always enough; the call reports the exact size otherwise
             for _ in range(2):
-                out = C.create_string_buffer(cap)
-                self._check(self._lib.cubit_disassemble(self._ctx, elf, only, int(frozen), out, cap, need, n_raw))
+                out = np.empty(cap, np.uint8)
+                self._check(self._lib.cubit_disassemble(self._ctx, elf, only, int(frozen), _ptr(out), cap, need, n_raw))
                 if need.value <= cap:
                     break
                 cap = need.value
         finally:
             self._lib.cubit_elf_free(elf)
-        text = out.value.decode()
+        text = str(out[:need.value - 1].data, "utf-8")
         return (text, int(n_raw.value)) if want_raw_count else text
 
     def assemble_listing(self, listing: str, kernel: str, want_failed: bool = False):
