@@ -316,8 +316,10 @@ struct cubit::DeviceState {
     // Grow-only staging for the host-memory paths.
     void* stage = nullptr;
     uint64_t stage_bytes = 0;
-    cudaStream_t stream = nullptr, stream2 = nullptr;
-    cudaEvent_t event = nullptr;
+    // Pinned slots of the host-memory paths, grow-only as well (at most three slots of 14 MiB).
+    uint8_t* pin = nullptr;
+    uint64_t pin_bytes = 0;
+    cudaStream_t stream = nullptr, stream2 = nullptr, stream3 = nullptr;
     std::mutex stage_mu;
     // Stream generator tables, one per (mix, seed).
     std::map<std::pair<uint32_t, uint64_t>, SynthView> synth;
@@ -391,9 +393,10 @@ void release_device(DeviceState* d) {
     if (d->counters) cudaFree(d->counters);
     if (d->stage) cudaFree(d->stage);
     if (d->stream) cudaStreamDestroy(d->stream);
+    if (d->pin) cudaFreeHost(d->pin);
     if (d->stream2) cudaStreamDestroy(d->stream2);
-    if (d->event) cudaEventDestroy(d->event);
-    d->counters = nullptr; d->stage = nullptr; d->stream = d->stream2 = nullptr; d->event = nullptr;
+    if (d->stream3) cudaStreamDestroy(d->stream3);
+    d->counters = nullptr; d->stage = nullptr; d->pin = nullptr; d->stream = d->stream2 = d->stream3 = nullptr;
 }
 
 std::string bundled_table_path() {
@@ -466,7 +469,7 @@ int init_device(const FlatTable& ft, DeviceState* d) {
     for (int s = 0; s < kCounterSlots; ++s) d->free_counter_slots.push_back(s);
     CU_TRY(c, cudaStreamCreateWithFlags(&d->stream, cudaStreamNonBlocking));
     CU_TRY(c, cudaStreamCreateWithFlags(&d->stream2, cudaStreamNonBlocking));
-    CU_TRY(c, cudaEventCreateWithFlags(&d->event, cudaEventDisableTiming));
+    CU_TRY(c, cudaStreamCreateWithFlags(&d->stream3, cudaStreamNonBlocking));
     return CUBIT_OK;
 }
 
@@ -601,103 +604,235 @@ void shard_range(uint64_t n, size_t g, size_t k, uint64_t* begin, uint64_t* end)
     *end = *begin + n / g + (k < n % g ? 1 : 0);
 }
 
-constexpr uint64_t kChunkWords = 1ull << 22;   // host paths stream the batch in 4 Mi-word chunks
-
 uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }
 
-// One chunk of a host batch on its way through the device: the stream it is queued on, its half
-// of the staging area, the first item and the number of items, and the counter slot of the call.
-struct ChunkIO {
-    cudaStream_t stream;
-    uint8_t* stage;
-    uint64_t at, items;
-    unsigned long long* counters;
+// ---- host batches --------------------------------------------------------------------------------
+//
+// A copy straight from or to pageable memory runs at 11 - 20 GB/s (the driver stages it through a small buffer with one
+// thread), and at 5 GB/s into pages that nobody has touched yet; pinned memory moves at 52 - 57 GB/s each way.  So the batch
+// goes through a ring of pinned slots: the context's host threads copy the caller's planes in and out piece by piece
+// (54 - 64 GB/s with four or more of them, page faults included on distinct pages at once), while the GPU works on the
+// slots between.  Small batches are not copied to the device at all: the kernel reads and writes the slot over the bus
+// (50 GB/s, both directions together), which leaves one launch where ten copies and a launch were.  The caller's planes that
+// are pinned themselves are not copied on the host; a batch of which all are uses the ring on the device only.
+//
+// One plane of a batch: item i is `bytes` bytes at host + i * bytes.
+struct HostPlane {
+    uint8_t* host;
+    uint32_t bytes;
+    enum Kind : uint8_t {
+        Plain,
+        Source,      // output that is a copy of the input words (never leaves the host)
+        Ctrl,        // ctrl words of a decode: counted as they are copied out
+        Status,      // roundtrip status bytes: likewise
+    } kind = Plain;
+    bool pinned = false;
 };
 
-// Streams items [begin, end) of a host batch through one device.  The range is cut into chunks
-// that alternate between two halves of the staging area and two streams, so the copy-in of one
-// chunk, the kernel of another and the copy-out of a third overlap (the PCIe link is full
-// duplex); with pinned host buffers every copy is asynchronous.  `body` queues the copies and
-// the launch of one chunk on the chunk's stream and returns the first CUDA error it met.
-// The caller holds the device's staging lock and has made the device current.  Whatever fails,
-// nothing is left running on either stream when this returns.
-template <typename Body>
-int pipeline_host_range(cubit_ctx* ctx, DeviceState* d, uint64_t begin, uint64_t end, uint64_t chunk, uint64_t half,
-                        cubit_counts* counts, const char* what, Body body) {
-    const bool two = end - begin > chunk;
-    int rc = ensure_stage(ctx, d, two ? 2 * half : half);
-    if (rc) return rc;
-    int slot = -1;
-    unsigned long long* dc = nullptr;
-    if (counts) {
-        slot = take_counter_slot(d);
-        if (slot < 0) return fail(ctx, CUBIT_ERR_NOMEM, "too many counted calls in flight on one device");
-        dc = d->counters + (size_t)slot * CNT_WORDS;
-    }
-    cudaStream_t streams[2] = {d->stream, d->stream2};
-    cudaError_t e = cudaSuccess;
-    if (dc) {
-        e = cudaMemsetAsync(dc, 0, sizeof(unsigned long long) * CNT_WORDS, streams[0]);
-        if (e == cudaSuccess) e = cudaEventRecord(d->event, streams[0]);
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(streams[1], d->event, 0);
-    }
-    uint64_t k = 0;
-    for (uint64_t at = begin; at < end && e == cudaSuccess; at += chunk, ++k)
-        e = body(ChunkIO{streams[k & 1], (uint8_t*)d->stage + (k & 1) * half, at, std::min(chunk, end - at), dc});
-    unsigned long long host[CNT_WORDS] = {0, 0, 0, 0, 0};
-    if (e == cudaSuccess) e = cudaStreamSynchronize(streams[1]);
-    if (e == cudaSuccess && dc) e = cudaMemcpyAsync(host, dc, sizeof host, cudaMemcpyDeviceToHost, streams[0]);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(streams[0]);
-    if (e != cudaSuccess) {   // nothing may still be using the staging area, the caller's buffers or the counter slot
-        cudaStreamSynchronize(streams[0]);
-        cudaStreamSynchronize(streams[1]);
+constexpr int kSlots = 3;                                // chunks in flight
+constexpr uint64_t kDirectWords = 1ull << 17;            // up to here the kernel works on the slots themselves
+constexpr uint64_t kDirectChunk = 1ull << 13;            // ... cut into chunks of at least this many
+constexpr uint64_t kSlotBytes = 14ull << 20;             // a slot of a large batch
+constexpr uint64_t kPinnedSlotBytes = 112ull << 20;      // ... when nothing is copied on the host
+constexpr uint64_t kPieceBytes = 512ull << 10;           // what one host thread copies at a time
+
+bool is_pinned(const void* p, uint64_t bytes) {
+    cudaPointerAttributes a, b;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess || cudaPointerGetAttributes(&b, (const uint8_t*)p + bytes - 1) != cudaSuccess) {
         cudaGetLastError();
+        return false;
     }
-    if (slot >= 0) give_counter_slot(d, slot);
-    if (e != cudaSuccess) return fail(ctx, CUBIT_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
-    if (counts) add_counts(counts, host);
+    return a.type == cudaMemoryTypeHost && b.type == cudaMemoryTypeHost;
+}
+
+// One chunk for the launch: where its planes are for the kernel, `stride` items apart within a group of planes.
+struct StagedChunk {
+    cudaStream_t stream;
+    uint64_t items, stride;
+    uint8_t* base;
+    const uint64_t* off;
+    uint8_t* plane(int k) const { return base + off[k]; }
+};
+
+int ensure_pinned(cubit_ctx* ctx, DeviceState* d, uint64_t bytes) {
+    if (d->pin_bytes >= bytes) return CUBIT_OK;
+    if (ctx->test_fail_alloc) return fail(ctx, CUBIT_ERR_NOMEM, "staging buffer allocation failed (injected by CUBIT_TEST_FAIL_ALLOC)");
+    if (d->pin) { CU_TRY(ctx, cudaFreeHost(d->pin)); d->pin = nullptr; d->pin_bytes = 0; }
+    CU_TRY(ctx, cudaHostAlloc((void**)&d->pin, bytes, cudaHostAllocPortable | cudaHostAllocMapped));
+    d->pin_bytes = bytes;
     return CUBIT_OK;
 }
 
-// Staging layout of one chunk of records: words, then the form, slot and ctrl planes.
-struct RecordStage {
-    uint64_t chunk, o_form, o_slots, o_ctrl, half;
-    explicit RecordStage(uint64_t items) {
-        chunk = std::min<uint64_t>(kChunkWords, std::max<uint64_t>(items, 1));
-        o_form = align_up(chunk * 16, 256);
-        o_slots = o_form + align_up(chunk * 2, 256);
-        o_ctrl = o_slots + chunk * 32;
-        half = align_up(o_ctrl + chunk * 4, 256);
-    }
-};
-
-// Queues the copy of one chunk's records from the staging area to host planes that are
-// `host_stride` records apart, record `at` of the call landing at `host_at`.
-cudaError_t records_to_host(const RecordStage& L, const ChunkIO& io, uint64_t host_at, uint64_t host_stride, uint16_t* form,
-                            uint32_t* slots, uint32_t* ctrl) {
-    cudaError_t e = cudaSuccess;
-    if (form) e = cudaMemcpyAsync(form + host_at, io.stage + L.o_form, io.items * 2, cudaMemcpyDeviceToHost, io.stream);
-    for (int p = 0; p < 8 && e == cudaSuccess && slots; ++p)
-        e = cudaMemcpyAsync(slots + (uint64_t)p * host_stride + host_at, io.stage + L.o_slots + (uint64_t)p * L.chunk * 4,
-                            io.items * 4, cudaMemcpyDeviceToHost, io.stream);
-    if (e == cudaSuccess && ctrl) e = cudaMemcpyAsync(ctrl + host_at, io.stage + L.o_ctrl, io.items * 4, cudaMemcpyDeviceToHost, io.stream);
-    return e;
+void count_ctrl(const uint32_t* c, uint64_t n, std::atomic<uint64_t>* rejected, std::atomic<uint64_t>* ties) {
+    uint64_t r = 0, t = 0;
+    for (uint64_t i = 0; i < n; ++i) { r += (c[i] >> 30) != 0; t += (c[i] >> 28) & 1u; }
+    *rejected += r;
+    *ties += t;
 }
 
-// Host-memory decode of words [begin, end) on one device.
-int decode_host_range(cubit_ctx* ctx, DeviceState* d, const uint8_t* words, uint64_t n_total, uint64_t begin,
-                      uint64_t end, uint16_t* form, uint32_t* slots, uint32_t* ctrl, cubit_counts* counts) {
+// Runs items [begin, end) through one device.  planes[0, n_in) are inputs, planes[n_in, n_planes) outputs; `gather`
+// copies input words [at, at + items) to a buffer where the words are not one array (then planes[0].host is null).
+// `launch` queues the kernel of one chunk.  The caller holds the device's staging lock and has made the device current.
+// Whatever fails, nothing is left running when this returns.
+template <typename Gather, typename Launch>
+int staged_host_range(cubit_ctx* ctx, DeviceState* d, uint64_t begin, uint64_t end, HostPlane* planes, int n_in, int n_planes,
+                      cubit_counts* counts, const char* what, Gather gather, Launch launch) {
+    const uint64_t n = end - begin;
+    uint64_t item_bytes = 0;
+    for (int k = 0; k < n_planes; ++k)
+        if (planes[k].kind != HostPlane::Source) item_bytes += planes[k].bytes;
+    const bool direct = n <= kDirectWords;
+    bool all_pinned = !direct;
+    for (int k = 0; k < n_planes && !direct; ++k) {
+        planes[k].pinned = planes[k].host && planes[k].kind != HostPlane::Source &&
+                           is_pinned(planes[k].host + begin * planes[k].bytes, n * planes[k].bytes);
+        all_pinned &= planes[k].pinned;
+    }
+    // A few chunks even of a small batch, so that copying in, the kernel and copying out overlap.
+    const uint64_t most = direct ? kDirectWords : std::max<uint64_t>((all_pinned ? kPinnedSlotBytes : kSlotBytes) / item_bytes, 1024);
+    const uint64_t chunk = std::min(most, std::max<uint64_t>(direct ? kDirectChunk : kDirectWords / 4, align_up((n + 3) / 4, 1024)));
+    const uint64_t slot_items = align_up(std::min(chunk, n), 64), slot_bytes = align_up(slot_items * item_bytes, 256);
+    const int slots = n > chunk ? kSlots : 1;
+    int rc = all_pinned ? (int)CUBIT_OK : ensure_pinned(ctx, d, slot_bytes * slots);
+    if (!rc && !direct) rc = ensure_stage(ctx, d, slot_bytes * slots);
+    if (rc) return rc;
+
+    struct InFlight { uint64_t at, items, stride; uint64_t off[16]; uint8_t* pin; };
+    InFlight flight[kSlots];
+    cudaStream_t streams[kSlots] = {d->stream, d->stream2, d->stream3};
+    std::atomic<uint64_t> rejected{0}, ties{0}, exact{0};
+    struct Piece { int plane; uint64_t first, items; };
+    std::vector<Piece> pieces;
+    const auto cut = [&](const InFlight& f, int from, int to) {
+        pieces.clear();
+        uint64_t bytes = 0;
+        for (int k = from; k < to; ++k) {
+            if (planes[k].pinned && !(counts && planes[k].kind != HostPlane::Plain)) continue;
+            const uint64_t per = std::max<uint64_t>(64, kPieceBytes / planes[k].bytes);
+            for (uint64_t i = 0; i < f.items; i += per) pieces.push_back(Piece{k, i, std::min(per, f.items - i)});
+            bytes += f.items * planes[k].bytes;
+        }
+        return bytes;
+    };
+    const auto copy_all = [&](uint64_t bytes, auto copy) {
+        if (bytes < (64u << 10)) for (const Piece& p : pieces) copy(p);
+        else ctx->pool.run(pieces.size(), [&](size_t i) { copy(pieces[i]); });
+    };
+    const auto finish = [&](const InFlight& f) {
+        copy_all(cut(f, n_in, n_planes), [&](const Piece& p) {
+            const HostPlane& h = planes[p.plane];
+            uint8_t* to = h.host + (f.at + p.first) * h.bytes;
+            if (h.kind == HostPlane::Source) return gather(f.at + p.first, p.items, to);
+            const uint8_t* from = h.pinned ? to : f.pin + f.off[p.plane] + p.first * h.bytes;
+            if (!h.pinned) memcpy(to, from, p.items * h.bytes);
+            if (h.kind == HostPlane::Ctrl && counts) count_ctrl((const uint32_t*)from, p.items, &rejected, &ties);
+            if (h.kind == HostPlane::Status && counts) {
+                uint64_t e = 0, r = 0;
+                for (uint64_t i = 0; i < p.items; ++i) { e += from[i] == RT_EXACT; r += from[i] == RT_REJECTED; }
+                exact += e;
+                rejected += r;
+            }
+        });
+    };
+    cudaError_t e = cudaSuccess;
+    uint64_t queued = 0, done = 0;
+    for (uint64_t at = begin; at < end && e == cudaSuccess; at += chunk, ++queued) {
+        const int slot = (int)(queued % (uint64_t)slots);
+        cudaStream_t stream = streams[slot];
+        InFlight& f = flight[slot];
+        if (queued - done == (uint64_t)slots) {
+            e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess) break;
+            finish(f);
+            ++done;
+        }
+        f.at = at; f.items = std::min(chunk, end - at);
+        f.stride = align_up(f.items, 64);
+        f.pin = d->pin + (uint64_t)slot * slot_bytes;
+        uint64_t off = 0;
+        for (int k = 0; k < n_planes; ++k) {
+            f.off[k] = off;
+            if (planes[k].kind != HostPlane::Source) off += f.stride * planes[k].bytes;
+        }
+        copy_all(cut(f, 0, n_in), [&](const Piece& p) {
+            const HostPlane& h = planes[p.plane];
+            uint8_t* to = f.pin + f.off[p.plane] + p.first * h.bytes;
+            if (h.host) memcpy(to, h.host + (at + p.first) * h.bytes, p.items * h.bytes);
+            else gather(at + p.first, p.items, to);
+        });
+        uint8_t* const dev = direct ? f.pin : (uint8_t*)d->stage + (uint64_t)slot * slot_bytes;
+        // Neighbouring planes that are staged move with one copy; the caller's own pinned planes each with one.
+        const auto move = [&](int from, int to, bool in) {
+            for (int k = from; k < to && e == cudaSuccess;) {
+                const HostPlane& h = planes[k];
+                if (h.kind == HostPlane::Source) { ++k; continue; }
+                if (h.pinned) {
+                    uint8_t* host = h.host + at * h.bytes;
+                    uint8_t* there = dev + f.off[k];
+                    e = in ? cudaMemcpyAsync(there, host, f.items * h.bytes, cudaMemcpyHostToDevice, stream)
+                           : cudaMemcpyAsync(host, there, f.items * h.bytes, cudaMemcpyDeviceToHost, stream);
+                    ++k;
+                    continue;
+                }
+                int last = k;
+                while (last + 1 < to && !planes[last + 1].pinned && planes[last + 1].kind != HostPlane::Source) ++last;
+                const uint64_t bytes = f.off[last] + f.items * planes[last].bytes - f.off[k];
+                e = in ? cudaMemcpyAsync(dev + f.off[k], f.pin + f.off[k], bytes, cudaMemcpyHostToDevice, stream)
+                       : cudaMemcpyAsync(f.pin + f.off[k], dev + f.off[k], bytes, cudaMemcpyDeviceToHost, stream);
+                k = last + 1;
+            }
+        };
+        if (!direct) move(0, n_in, true);
+        if (e == cudaSuccess) {
+            launch(StagedChunk{stream, f.items, f.stride, dev, f.off});
+            e = cudaGetLastError();
+        }
+        if (!direct && e == cudaSuccess) move(n_in, n_planes, false);
+    }
+    for (; done < queued && e == cudaSuccess; ++done) {
+        const int slot = (int)(done % (uint64_t)slots);
+        e = cudaStreamSynchronize(streams[slot]);
+        if (e == cudaSuccess) finish(flight[slot]);
+    }
+    if (e != cudaSuccess) {   // nothing may still be using the slots, the staging area or the caller's buffers
+        for (cudaStream_t s : streams) cudaStreamSynchronize(s);
+        cudaGetLastError();
+        return fail(ctx, CUBIT_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    }
+    if (counts) {
+        bool status = false;
+        for (int k = n_in; k < n_planes; ++k) status |= planes[k].kind == HostPlane::Status;
+        counts->n_rejected += rejected;
+        if (status) { counts->n_exact += exact; counts->n_mismatch += n - exact - rejected; }
+        else { counts->n_decoded += n - rejected; counts->n_tie += ties; }
+    }
+    return CUBIT_OK;
+}
+
+// The planes of `n_total` records: form, eight slots, ctrl.
+void add_record_planes(HostPlane* planes, int* n, uint64_t n_total, const uint16_t* form, const uint32_t* slots, const uint32_t* ctrl,
+                       HostPlane::Kind ctrl_kind) {
+    planes[(*n)++] = HostPlane{(uint8_t*)form, 2};
+    for (uint64_t s = 0; s < 8; ++s) planes[(*n)++] = HostPlane{(uint8_t*)(slots + s * n_total), 4};
+    planes[(*n)++] = HostPlane{(uint8_t*)ctrl, 4, ctrl_kind};
+}
+const auto kNoGather = [](uint64_t, uint64_t, uint8_t*) {};
+
+// Host-memory decode of words [begin, end) on one device.  `gather` fetches words when they are not one array; `raw`,
+// when given, receives them.
+template <typename Gather>
+int decode_host_range(cubit_ctx* ctx, DeviceState* d, const uint8_t* words, Gather gather, uint64_t n_total, uint64_t begin, uint64_t end,
+                      uint16_t* form, uint32_t* slots, uint32_t* ctrl, uint8_t* raw, cubit_counts* counts, const char* what) {
     std::lock_guard<std::mutex> g(d->stage_mu);
     CU_TRY(ctx, cudaSetDevice(d->device));
-    const RecordStage L(end - begin);
-    return pipeline_host_range(ctx, d, begin, end, L.chunk, L.half, counts, "host decode", [&](const ChunkIO& io) {
-        cudaError_t e = cudaMemcpyAsync(io.stage, words + io.at * 16, io.items * 16, cudaMemcpyHostToDevice, io.stream);
-        if (e != cudaSuccess) return e;
-        launch_decode(d, io.stream, (const uint4*)io.stage, io.items, (uint16_t*)(io.stage + L.o_form),
-                      (uint32_t*)(io.stage + L.o_slots), L.chunk, (uint32_t*)(io.stage + L.o_ctrl), io.counters);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = records_to_host(L, io, io.at, n_total, form, slots, ctrl);
-        return e;
+    HostPlane planes[12];
+    int n = 0;
+    planes[n++] = HostPlane{(uint8_t*)words, 16};
+    add_record_planes(planes, &n, n_total, form, slots, ctrl, HostPlane::Ctrl);
+    if (raw) planes[n++] = HostPlane{raw, 16, HostPlane::Source};
+    return staged_host_range(ctx, d, begin, end, planes, 1, n, counts, what, gather, [d](const StagedChunk& c) {
+        launch_decode(d, c.stream, (const uint4*)c.plane(0), c.items, (uint16_t*)c.plane(1), (uint32_t*)c.plane(2), c.stride,
+                      (uint32_t*)c.plane(10), nullptr);
     });
 }
 
@@ -705,19 +840,13 @@ int encode_host_range(cubit_ctx* ctx, DeviceState* d, const uint16_t* form, cons
                       uint64_t n_total, uint64_t begin, uint64_t end, uint8_t* words) {
     std::lock_guard<std::mutex> g(d->stage_mu);
     CU_TRY(ctx, cudaSetDevice(d->device));
-    const RecordStage L(end - begin);
-    return pipeline_host_range(ctx, d, begin, end, L.chunk, L.half, nullptr, "host encode", [&](const ChunkIO& io) {
-        cudaError_t e = cudaMemcpyAsync(io.stage + L.o_form, form + io.at, io.items * 2, cudaMemcpyHostToDevice, io.stream);
-        for (int k = 0; k < 8 && e == cudaSuccess; ++k)
-            e = cudaMemcpyAsync(io.stage + L.o_slots + (uint64_t)k * L.chunk * 4, slots + (uint64_t)k * n_total + io.at,
-                                io.items * 4, cudaMemcpyHostToDevice, io.stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(io.stage + L.o_ctrl, ctrl + io.at, io.items * 4, cudaMemcpyHostToDevice, io.stream);
-        if (e != cudaSuccess) return e;
-        launch_encode(d, io.stream, (const uint16_t*)(io.stage + L.o_form), (const uint32_t*)(io.stage + L.o_slots), L.chunk,
-                      (const uint32_t*)(io.stage + L.o_ctrl), io.items, (uint4*)io.stage);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(words + io.at * 16, io.stage, io.items * 16, cudaMemcpyDeviceToHost, io.stream);
-        return e;
+    HostPlane planes[11];
+    int n = 0;
+    add_record_planes(planes, &n, n_total, form, slots, ctrl, HostPlane::Plain);
+    planes[n++] = HostPlane{words, 16};
+    return staged_host_range(ctx, d, begin, end, planes, n - 1, n, nullptr, "host encode", kNoGather, [d](const StagedChunk& c) {
+        launch_encode(d, c.stream, (const uint16_t*)c.plane(0), (const uint32_t*)c.plane(1), c.stride, (const uint32_t*)c.plane(9),
+                      c.items, (uint4*)c.plane(10));
     });
 }
 
@@ -725,15 +854,9 @@ int roundtrip_host_range(cubit_ctx* ctx, DeviceState* d, const uint8_t* words, u
                          uint8_t* status, cubit_counts* counts) {
     std::lock_guard<std::mutex> g(d->stage_mu);
     CU_TRY(ctx, cudaSetDevice(d->device));
-    const uint64_t chunk = std::min<uint64_t>(kChunkWords, std::max<uint64_t>(end - begin, 1));
-    const uint64_t o_status = align_up(chunk * 16, 256), half = align_up(o_status + chunk, 256);
-    return pipeline_host_range(ctx, d, begin, end, chunk, half, counts, "host roundtrip", [&](const ChunkIO& io) {
-        cudaError_t e = cudaMemcpyAsync(io.stage, words + io.at * 16, io.items * 16, cudaMemcpyHostToDevice, io.stream);
-        if (e != cudaSuccess) return e;
-        launch_roundtrip(d, io.stream, (const uint4*)io.stage, io.items, io.stage + o_status, io.counters);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(status + io.at, io.stage + o_status, io.items, cudaMemcpyDeviceToHost, io.stream);
-        return e;
+    HostPlane planes[2] = {HostPlane{(uint8_t*)words, 16}, HostPlane{status, 1, HostPlane::Status}};
+    return staged_host_range(ctx, d, begin, end, planes, 1, 2, counts, "host roundtrip", kNoGather, [d](const StagedChunk& c) {
+        launch_roundtrip(d, c.stream, (const uint4*)c.plane(0), c.items, c.plane(1), nullptr);
     });
 }
 
@@ -952,7 +1075,8 @@ extern "C" int cubit_decode_batch(cubit_ctx* ctx, const void* words, uint64_t n,
         uint64_t b, e;
         shard_range(n, g, k, &b, &e);
         if (b == e) return (int)CUBIT_OK;
-        return decode_host_range(ctx, ctx->devs[k].get(), (const uint8_t*)words, n, b, e, form, slots, ctrl, part);
+        return decode_host_range(ctx, ctx->devs[k].get(), (const uint8_t*)words, kNoGather, n, b, e, form, slots, ctrl, nullptr, part,
+                                 "host decode");
     });
 } catch (...) {
     return translate_exception(ctx);
@@ -1044,16 +1168,19 @@ extern "C" int cubit_synth_batch(cubit_ctx* ctx, uint32_t mix, uint64_t seed, ui
     if (rc) return rc;
     std::lock_guard<std::mutex> lock(d->stage_mu);
     CU_TRY(ctx, cudaSetDevice(d->device));
-    const RecordStage L(n);
-    return pipeline_host_range(ctx, d, 0, n, L.chunk, L.half, nullptr, "host stream generator", [&](const ChunkIO& io) {
-        synth_kernel<<<grid_for(d, io.items), kBlock, 0, io.stream>>>(d->view, g, first + io.at, io.items, (uint4*)io.stage,
-                                                                       (uint16_t*)(io.stage + L.o_form), (uint32_t*)(io.stage + L.o_slots),
-                                                                       L.chunk, (uint32_t*)(io.stage + L.o_ctrl));
-        cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess && words)
-            e = cudaMemcpyAsync((uint8_t*)words + io.at * 16, io.stage, io.items * 16, cudaMemcpyDeviceToHost, io.stream);
-        if (e == cudaSuccess) e = records_to_host(L, io, io.at, n, form, slots, ctrl);
-        return e;
+    HostPlane planes[11];
+    int n_planes = 0, at[4] = {-1, -1, -1, -1};   // words, form, slots, ctrl among them
+    if (words) { at[0] = n_planes; planes[n_planes++] = HostPlane{(uint8_t*)words, 16}; }
+    if (form) { at[1] = n_planes; planes[n_planes++] = HostPlane{(uint8_t*)form, 2}; }
+    if (slots) { at[2] = n_planes; for (uint64_t p = 0; p < 8; ++p) planes[n_planes++] = HostPlane{(uint8_t*)(slots + p * n), 4}; }
+    if (ctrl) { at[3] = n_planes; planes[n_planes++] = HostPlane{(uint8_t*)ctrl, 4}; }
+    if (!n_planes) return CUBIT_OK;
+    uint64_t next = first;   // chunks are launched in order
+    return staged_host_range(ctx, d, 0, n, planes, 0, n_planes, nullptr, "host stream generator", kNoGather, [&](const StagedChunk& c) {
+        const auto plane = [&](int k) { return at[k] < 0 ? nullptr : c.plane(at[k]); };
+        synth_kernel<<<grid_for(d, c.items), kBlock, 0, c.stream>>>(d->view, g, next, c.items, (uint4*)plane(0), (uint16_t*)plane(1),
+                                                                    (uint32_t*)plane(2), c.stride, (uint32_t*)plane(3));
+        next += c.items;
     });
 } catch (...) {
     return translate_exception(ctx);
@@ -1200,29 +1327,19 @@ extern "C" int cubit_decode_elf(cubit_ctx* ctx, const cubit_elf* elf, const uint
         uint64_t b, e;
         shard_range(total, g, k, &b, &e);
         if (b == e) return (int)CUBIT_OK;
-        DeviceState* d = ctx->devs[k].get();
-        std::lock_guard<std::mutex> lock(d->stage_mu);
-        CU_TRY(ctx, cudaSetDevice(d->device));
-        // The device's share of the records goes through the staging area chunk by chunk: each chunk gathers
-        // its part of the text ranges, is decoded by one launch and copied out while the next one comes in.
-        const RecordStage L(e - b);
-        return pipeline_host_range(ctx, d, b, e, L.chunk, L.half, part, "cubin decode", [&](const ChunkIO& io) {
-            cudaError_t err = cudaSuccess;
-            for (const Range& r : ranges) {
-                const uint64_t lo = std::max(io.at, r.rec), hi = std::min(io.at + io.items, r.rec + r.words);
-                if (lo >= hi) continue;
-                const uint8_t* src = elf->bytes + r.file_off + (lo - r.rec) * 16;
-                err = cudaMemcpyAsync(io.stage + (lo - io.at) * 16, src, (hi - lo) * 16, cudaMemcpyHostToDevice, io.stream);
-                if (err != cudaSuccess) return err;
+        // The words of a range of records, section by section.
+        const auto gather = [&](uint64_t at, uint64_t items, uint8_t* to) {
+            auto r = std::upper_bound(ranges.begin(), ranges.end(), at, [](uint64_t v, const Range& x) { return v < x.rec; }) - 1;
+            for (; items; ++r) {
+                const uint64_t skip = at - r->rec, take = std::min(items, r->words - skip);
+                memcpy(to, elf->bytes + r->file_off + skip * 16, take * 16);
+                at += take; items -= take; to += take * 16;
             }
-            launch_decode(d, io.stream, (const uint4*)io.stage, io.items, (uint16_t*)(io.stage + L.o_form),
-                          (uint32_t*)(io.stage + L.o_slots), L.chunk, (uint32_t*)(io.stage + L.o_ctrl), io.counters);
-            err = cudaGetLastError();
-            if (err == cudaSuccess) err = records_to_host(L, io, io.at, capacity, form, slots, ctrl);
-            if (err == cudaSuccess && raw_words)
-                err = cudaMemcpyAsync((uint8_t*)raw_words + io.at * 16, io.stage, io.items * 16, cudaMemcpyDeviceToHost, io.stream);
-            return err;
-        });
+        };
+        // One text range is an array of words like any other.
+        const uint8_t* words = ranges.size() == 1 ? elf->bytes + ranges[0].file_off : nullptr;
+        return decode_host_range(ctx, ctx->devs[k].get(), words, gather, capacity, b, e, form, slots, ctrl, (uint8_t*)raw_words, part,
+                                 "cubin decode");
     });
 } catch (...) {
     return translate_exception(ctx);
