@@ -17,6 +17,7 @@ import numpy as np
 
 from . import _native
 from ._native import Counts, VariantInfo
+from ._results import ResultPool
 
 MEM_HOST, MEM_DEVICE = 0, 1
 MIX_UNIFORM, MIX_ZIPF, MIX_FAMILY = 0, 1, 2
@@ -93,11 +94,13 @@ class Codec:
             raise CubitError(rc, self._lib.cubit_last_error(None).decode())
         self.devices = tuple(devices)
         self._meta: dict[int, VariantMeta] = {}
+        self._results = ResultPool()
 
     def close(self):
         if getattr(self, "_ctx", None):
             self._lib.cubit_ctx_destroy(self._ctx)
             self._ctx = None
+            self._results.clear()
 
     def __del__(self):
         try:
@@ -149,11 +152,16 @@ class Codec:
             raise ValueError("word buffer length is not a multiple of 16 bytes")
         return w.reshape(-1, 16)
 
+    def _record_arrays(self, n: int):
+        """Arrays for n records: form, slots, ctrl."""
+        new = self._results.empty
+        return new(n, np.uint16), new((8, n), np.uint32), new(n, np.uint32)
+
     def decode_batch(self, words):
         """(n,16) uint8 little-endian words -> (form u16[n], slots u32[8,n], ctrl u32[n], counts)."""
         w = self._words(words)
         n = len(w)
-        form = np.empty(n, np.uint16); slots = np.empty((8, n), np.uint32); ctrl = np.empty(n, np.uint32)
+        form, slots, ctrl = self._record_arrays(n)
         counts = Counts()
         self._check(self._lib.cubit_decode_batch(self._ctx, _ptr(w), n, _ptr(form), _ptr(slots), _ptr(ctrl),
                                                  C.byref(counts), MEM_HOST, None))
@@ -167,7 +175,7 @@ class Codec:
         serialises them with one lock per GPU, so they are safe but do not run in parallel."""
         w = self._words(words)
         n = len(w)
-        form = np.empty(n, np.uint16); slots = np.empty((8, n), np.uint32); ctrl = np.empty(n, np.uint32)
+        form, slots, ctrl = self._record_arrays(n)
         counts = Counts()
         self._check(self._lib.cubit_decode_batch_static(self._ctx, device_slot, _ptr(w), n, _ptr(form), _ptr(slots),
                                                         _ptr(ctrl), C.byref(counts)))
@@ -179,14 +187,14 @@ class Codec:
         n = len(form)
         if slots.shape != (8, n) or ctrl.shape != (n,):
             raise ValueError("slots must be (8, n) and ctrl (n,)")
-        words = np.empty((n, 16), np.uint8)
+        words = self._results.empty((n, 16), np.uint8)
         self._check(self._lib.cubit_encode_batch(self._ctx, _ptr(form), _ptr(slots), _ptr(ctrl), n, _ptr(words),
                                                  MEM_HOST, None))
         return words
 
     def roundtrip_batch(self, words):
         w = self._words(words)
-        status = np.empty(len(w), np.uint8)
+        status = self._results.empty(len(w), np.uint8)
         counts = Counts()
         self._check(self._lib.cubit_roundtrip_batch(self._ctx, _ptr(w), len(w), _ptr(status), C.byref(counts),
                                                     MEM_HOST, None))
@@ -194,8 +202,8 @@ class Codec:
 
     def synth(self, mix: int, seed: int, n: int, noise_ppm: int = 0, first: int = 0):
         """Words [first, first+n) of a seeded synthetic stream and the generator's records."""
-        words = np.empty((n, 16), np.uint8); form = np.empty(n, np.uint16)
-        slots = np.empty((8, n), np.uint32); ctrl = np.empty(n, np.uint32)
+        words = self._results.empty((n, 16), np.uint8)
+        form, slots, ctrl = self._record_arrays(n)
         self._check(self._lib.cubit_synth_batch(self._ctx, mix, seed, noise_ppm, first, n, _ptr(words), _ptr(form),
                                                 _ptr(slots), _ptr(ctrl), MEM_HOST, None))
         return words, form, slots, ctrl
@@ -409,8 +417,8 @@ class Codec:
             self._check(self._lib.cubit_decode_elf(self._ctx, elf, _ptr(indices), k, _ptr(word_start), 0, None, None,
                                                    None, None, None))
             total = int(word_start[k])
-            form = np.empty(total, np.uint16); slots = np.empty((8, total), np.uint32); ctrl = np.empty(total, np.uint32)
-            raw = np.empty((total, 16), np.uint8) if want_raw else None
+            form, slots, ctrl = self._record_arrays(total)
+            raw = self._results.empty((total, 16), np.uint8) if want_raw else None
             counts = Counts()
             self._check(self._lib.cubit_decode_elf(self._ctx, elf, _ptr(indices), k, _ptr(word_start), total, _ptr(form),
                                                    _ptr(slots), _ptr(ctrl), _ptr(raw), C.byref(counts)))
@@ -476,7 +484,7 @@ class Codec:
                 total += size.value // 16
             cap = 112 * total + 512 * n_text + 64   # nearly always enough; the call reports the exact size otherwise
             for _ in range(2):
-                out = np.empty(cap, np.uint8)
+                out = self._results.empty(cap, np.uint8)
                 self._check(self._lib.cubit_disassemble(self._ctx, elf, only, int(frozen), _ptr(out), cap, need, n_raw))
                 if need.value <= cap:
                     break

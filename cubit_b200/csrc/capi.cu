@@ -630,11 +630,11 @@ struct HostPlane {
 };
 
 constexpr int kSlots = 3;                                // chunks in flight
-constexpr uint64_t kDirectWords = 1ull << 17;            // up to here the kernel works on the slots themselves
-constexpr uint64_t kDirectChunk = 1ull << 13;            // ... cut into chunks of at least this many
+constexpr uint64_t kDirectWords = 1ull << 18;            // up to here the kernel works on the slots themselves
+constexpr uint64_t kDirectChunk = 1ull << 14;            // ... cut into chunks of at least this many
 constexpr uint64_t kSlotBytes = 14ull << 20;             // a slot of a large batch
 constexpr uint64_t kPinnedSlotBytes = 112ull << 20;      // ... when nothing is copied on the host
-constexpr uint64_t kPieceBytes = 512ull << 10;           // what one host thread copies at a time
+constexpr uint64_t kPieceBytes = 64ull << 10;            // what one host thread copies at a time (256 KiB: 5 % slower)
 
 bool is_pinned(const void* p, uint64_t bytes) {
     cudaPointerAttributes a, b;
@@ -663,11 +663,33 @@ int ensure_pinned(cubit_ctx* ctx, DeviceState* d, uint64_t bytes) {
     return CUBIT_OK;
 }
 
+// What the counters of a call say, from the records that it copies out (a few percent of the copy).
 void count_ctrl(const uint32_t* c, uint64_t n, std::atomic<uint64_t>* rejected, std::atomic<uint64_t>* ties) {
-    uint64_t r = 0, t = 0;
-    for (uint64_t i = 0; i < n; ++i) { r += (c[i] >> 30) != 0; t += (c[i] >> 28) & 1u; }
+    uint32_t r = 0, t = 0;
+    for (uint64_t i = 0; i < n; ++i) { r += ((c[i] >> 30) | (c[i] >> 31)) & 1u; t += (c[i] >> 28) & 1u; }
     *rejected += r;
     *ties += t;
+}
+// Status bytes are 0, 1 or 2 (RT_*), so bit 0 and bit 1 of each byte are the two counts: eight bytes at a time.
+void count_status(const uint8_t* s, uint64_t n, std::atomic<uint64_t>* mismatch, std::atomic<uint64_t>* rejected) {
+    static_assert(RT_EXACT == 0 && RT_MISMATCH == 1 && RT_REJECTED == 2, "counted by bit");
+    const uint64_t ones = 0x0101010101010101ull, even = 0x00FF00FF00FF00FFull;
+    uint64_t m = 0, r = 0, i = 0;
+    while (n - i >= 8) {
+        uint64_t acc_m = 0, acc_r = 0;
+        for (int k = 0; k < 255 && n - i >= 8; ++k, i += 8) {   // no byte of the sums overflows
+            uint64_t w;
+            memcpy(&w, s + i, 8);
+            acc_m += w & ones;
+            acc_r += (w >> 1) & ones;
+        }
+        const auto add = [&](uint64_t a) { return (((a & even) + ((a >> 8) & even)) * 0x0001000100010001ull) >> 48; };
+        m += add(acc_m);
+        r += add(acc_r);
+    }
+    for (; i < n; ++i) { m += s[i] & 1u; r += s[i] >> 1; }
+    *mismatch += m;
+    *rejected += r;
 }
 
 // Runs items [begin, end) through one device.  planes[0, n_in) are inputs, planes[n_in, n_planes) outputs; `gather`
@@ -700,7 +722,8 @@ int staged_host_range(cubit_ctx* ctx, DeviceState* d, uint64_t begin, uint64_t e
     struct InFlight { uint64_t at, items, stride; uint64_t off[16]; uint8_t* pin; };
     InFlight flight[kSlots];
     cudaStream_t streams[kSlots] = {d->stream, d->stream2, d->stream3};
-    std::atomic<uint64_t> rejected{0}, ties{0}, exact{0};
+    std::atomic<uint64_t> rejected{0}, ties{0}, mismatch{0};
+    const WorkPool::Awake awake(ctx->pool);
     struct Piece { int plane; uint64_t first, items; };
     std::vector<Piece> pieces;
     const auto cut = [&](const InFlight& f, int from, int to) {
@@ -708,7 +731,7 @@ int staged_host_range(cubit_ctx* ctx, DeviceState* d, uint64_t begin, uint64_t e
         uint64_t bytes = 0;
         for (int k = from; k < to; ++k) {
             if (planes[k].pinned && !(counts && planes[k].kind != HostPlane::Plain)) continue;
-            const uint64_t per = std::max<uint64_t>(64, kPieceBytes / planes[k].bytes);
+            const uint64_t per = std::max<uint64_t>(64, kPieceBytes / std::max(planes[k].bytes, 4u));
             for (uint64_t i = 0; i < f.items; i += per) pieces.push_back(Piece{k, i, std::min(per, f.items - i)});
             bytes += f.items * planes[k].bytes;
         }
@@ -726,12 +749,7 @@ int staged_host_range(cubit_ctx* ctx, DeviceState* d, uint64_t begin, uint64_t e
             const uint8_t* from = h.pinned ? to : f.pin + f.off[p.plane] + p.first * h.bytes;
             if (!h.pinned) memcpy(to, from, p.items * h.bytes);
             if (h.kind == HostPlane::Ctrl && counts) count_ctrl((const uint32_t*)from, p.items, &rejected, &ties);
-            if (h.kind == HostPlane::Status && counts) {
-                uint64_t e = 0, r = 0;
-                for (uint64_t i = 0; i < p.items; ++i) { e += from[i] == RT_EXACT; r += from[i] == RT_REJECTED; }
-                exact += e;
-                rejected += r;
-            }
+            if (h.kind == HostPlane::Status && counts) count_status(from, p.items, &mismatch, &rejected);
         });
     };
     cudaError_t e = cudaSuccess;
@@ -803,7 +821,7 @@ int staged_host_range(cubit_ctx* ctx, DeviceState* d, uint64_t begin, uint64_t e
         bool status = false;
         for (int k = n_in; k < n_planes; ++k) status |= planes[k].kind == HostPlane::Status;
         counts->n_rejected += rejected;
-        if (status) { counts->n_exact += exact; counts->n_mismatch += n - exact - rejected; }
+        if (status) { counts->n_mismatch += mismatch; counts->n_exact += n - mismatch - rejected; }
         else { counts->n_decoded += n - rejected; counts->n_tie += ties; }
     }
     return CUBIT_OK;

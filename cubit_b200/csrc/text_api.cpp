@@ -252,6 +252,7 @@ extern "C" int cubit_text_encode(cubit_ctx* ctx, const char* text, uint32_t base
     if (!ctx) return CUBIT_ERR_INVALID;
     if (!text || !n_out) return fail(ctx, CUBIT_ERR_INVALID, "null argument");
     if (mode != CUBIT_TEXT_ONE && mode != CUBIT_TEXT_PROGRAM) return fail(ctx, CUBIT_ERR_INVALID, "unknown text mode");
+    const WorkPool::Awake awake(ctx->pool);
     const std::vector<ProgramRun> runs = lower_text(ctx, text, base_addr, mode);
     const uint64_t n = count_rows(runs);
     *n_out = n;
@@ -661,6 +662,7 @@ extern "C" int cubit_disassemble(cubit_ctx* ctx, const cubit_elf* elf, const cha
     if (!ctx) return CUBIT_ERR_INVALID;
     if (!elf || !needed) return fail(ctx, CUBIT_ERR_INVALID, "null argument");
     if (n_raw) *n_raw = 0;
+    const WorkPool::Awake awake(ctx->pool);
     std::vector<ElfSection> sections;
     try {
         sections = elf_sections(elf->bytes, elf->len);
@@ -952,6 +954,7 @@ extern "C" int cubit_patch_elf(cubit_ctx* ctx, const cubit_elf* elf, void* out, 
         if (stats) *stats = st;
         return CUBIT_OK;
     }
+    const WorkPool::Awake awake(ctx->pool);
     DecodedText code;
     int rc = code.decode(ctx, elf, all);
     if (rc) return rc;

@@ -26,8 +26,7 @@ public:
     ~WorkPool() {
         {
             std::lock_guard<std::mutex> g(mu_);
-            stop_ = true;
-            open_.fetch_add(1);   // ends the spinning
+            stop_.store(true);
         }
         cv_.notify_all();
         for (std::thread& t : threads_) t.join();
@@ -38,33 +37,35 @@ public:
     // Threads that can work on one job: the workers and the caller.
     unsigned width() const { return wanted_ + 1; }
 
+    // While one of these lives, workers without work keep looking for longer: a call that waits for the GPU between its
+    // jobs finds them awake (asleep, they cost a batch of 9 Mi words 3 of 8 ms).
+    class Awake {
+    public:
+        explicit Awake(WorkPool& pool) : pool_(pool) { pool_.awake_.fetch_add(1, std::memory_order_relaxed); }
+        ~Awake() { pool_.awake_.fetch_sub(1, std::memory_order_relaxed); }
+        Awake(const Awake&) = delete;
+        Awake& operator=(const Awake&) = delete;
+    private:
+        WorkPool& pool_;
+    };
+
     // Calls fn(piece) for every piece in [0, n), from several threads, and returns when all are done.  An exception is
     // rethrown here; with several, the one of the lowest piece.  May be called from several threads at once.
     template <typename Fn>
     void run(size_t n, Fn&& fn) {
-        if (n <= 1 || !wanted_) {
-            for (size_t i = 0; i < n; ++i) fn(i);
-            return;
-        }
         typedef typename std::remove_reference<Fn>::type Body;
         Job job;
         job.n = n;
         job.body = const_cast<void*>(static_cast<const void*>(&fn));
         job.call = [](void* body, size_t i) { (*static_cast<Body*>(body))(i); };
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            if (threads_.empty()) start();
-            jobs_.push_back(&job);
-            open_.fetch_add(1);
+        Slot* slot = n > 1 && wanted_ && started() ? publish(&job) : nullptr;
+        job.work(open_, slot != nullptr);
+        if (slot) {
+            // Nobody can join the job any more once it is withdrawn; those who did finish the pieces that they took.
+            slot->job.store(nullptr);
+            while (slot->users.load()) relax();
+            slot->taken.store(false, std::memory_order_release);
         }
-        cv_.notify_one();   // a woken worker wakes the next one
-        job.work(open_);
-        {
-            std::lock_guard<std::mutex> g(mu_);
-            jobs_.erase(std::find(jobs_.begin(), jobs_.end(), &job));
-        }
-        // Nobody can join the job any more; those who did finish the pieces that they took.
-        while (job.users.load(std::memory_order_acquire)) relax();
         if (job.error) std::rethrow_exception(job.error);
     }
 
@@ -87,13 +88,12 @@ private:
         size_t n = 0;
         void* body = nullptr;
         void (*call)(void*, size_t) = nullptr;
-        std::atomic<size_t> next{0};
-        std::atomic<unsigned> users{0};
+        alignas(64) std::atomic<size_t> next{0};
         std::atomic<bool> drained{false};
         std::mutex error_mu;
         std::exception_ptr error;
         size_t error_at = 0;
-        void work(std::atomic<int>& open) {
+        void work(std::atomic<int>& open, bool published) {
             for (size_t i; (i = next.fetch_add(1, std::memory_order_relaxed)) < n;) {
                 try {
                     call(body, i);
@@ -102,53 +102,89 @@ private:
                     if (!error || i < error_at) { error = std::current_exception(); error_at = i; }
                 }
             }
-            if (!drained.exchange(true)) open.fetch_sub(1);   // every piece is taken: nothing for anybody to join
+            if (published && !drained.exchange(true)) open.fetch_sub(1);   // every piece is taken: nothing for anybody to join
         }
     };
+    // Where a job is found.  A worker counts itself in before it looks whether the job is still there, the caller waits
+    // for the count after it has taken the job away: the job outlives everybody who works on it.
+    struct alignas(64) Slot {
+        std::atomic<bool> taken{false};
+        std::atomic<Job*> job{nullptr};
+        std::atomic<unsigned> users{0};
+    };
 
-    void start() {   // mu_ is held
-        for (unsigned k = 0; k < wanted_; ++k) {
+    bool started() {
+        if (started_.load(std::memory_order_acquire)) return true;
+        std::lock_guard<std::mutex> g(mu_);
+        for (unsigned k = (unsigned)threads_.size(); k < wanted_; ++k) {
             try {
                 threads_.emplace_back([this] { loop(); });
             } catch (const std::system_error&) {   // no more threads to be had: go on with those that there are
-                if (threads_.empty()) wanted_ = 0;
-                return;
+                wanted_ = k;
             }
         }
+        started_.store(true, std::memory_order_release);
+        return wanted_ > 0;
+    }
+
+    Slot* publish(Job* job) {   // null when too many jobs are open already: the caller does this one alone
+        for (Slot& s : slots_) {
+            if (s.taken.load(std::memory_order_relaxed) || s.taken.exchange(true)) continue;
+            open_.fetch_add(1);
+            s.job.store(job);
+            wake();
+            return &s;
+        }
+        return nullptr;
+    }
+    void wake() {   // one sleeper; it wakes the next
+        if (!sleeping_.load()) return;
+        std::lock_guard<std::mutex> g(mu_);
+        cv_.notify_one();
     }
 
     void loop() {
-        for (;;) {
-            Job* job = nullptr;
-            const auto until = std::chrono::steady_clock::now() + std::chrono::microseconds(kSpinMicros);
-            while (!job) {
+        while (!stop_.load(std::memory_order_relaxed)) {
+            if (join_one()) continue;
+            const auto from = std::chrono::steady_clock::now();
+            while (!open_.load(std::memory_order_relaxed) && !stop_.load(std::memory_order_relaxed)) {
                 for (int k = 0; k < 32 && !open_.load(std::memory_order_relaxed); ++k) relax();
-                const bool tired = std::chrono::steady_clock::now() > until;
-                if (!tired && !open_.load(std::memory_order_relaxed)) continue;
+                const auto most = std::chrono::microseconds(awake_.load(std::memory_order_relaxed) ? kAwakeMicros : kSpinMicros);
+                if (std::chrono::steady_clock::now() - from < most) continue;
                 std::unique_lock<std::mutex> g(mu_);
-                if (tired) cv_.wait(g, [this] { return stop_ || unfinished(); });
-                if (stop_) return;
-                if ((job = unfinished())) job->users.fetch_add(1, std::memory_order_relaxed);
+                sleeping_.fetch_add(1);
+                cv_.wait(g, [this] { return stop_.load() || open_.load() > 0; });
+                sleeping_.fetch_sub(1);
+                break;
             }
-            cv_.notify_one();
-            job->work(open_);
-            job->users.fetch_sub(1, std::memory_order_release);
         }
     }
-    Job* unfinished() const {
-        for (Job* j : jobs_)
-            if (j->next.load(std::memory_order_relaxed) < j->n) return j;
-        return nullptr;
+    bool join_one() {
+        for (Slot& s : slots_) {
+            if (!s.job.load(std::memory_order_relaxed)) continue;
+            s.users.fetch_add(1);
+            Job* const job = s.job.load();
+            const bool worth = job && job->next.load(std::memory_order_relaxed) < job->n;
+            if (worth) {
+                wake();
+                job->work(open_, true);
+            }
+            s.users.fetch_sub(1);
+            if (worth) return true;
+        }
+        return false;
     }
 
-    enum { kSpinMicros = 50 };
+    enum { kSpinMicros = 50, kAwakeMicros = 1000, kSlots = 8 };
     std::atomic<unsigned> wanted_;
     std::mutex mu_;
     std::condition_variable cv_;
     std::vector<std::thread> threads_;
-    std::vector<Job*> jobs_;
-    std::atomic<int> open_{0};   // jobs with pieces left to take: what idle workers look at without the lock
-    bool stop_ = false;
+    Slot slots_[kSlots];
+    std::atomic<int> open_{0};        // jobs with pieces left to take: what idle workers look at
+    std::atomic<int> sleeping_{0};
+    std::atomic<int> awake_{0};
+    std::atomic<bool> started_{false}, stop_{false};
 };
 
 }  // namespace cubit

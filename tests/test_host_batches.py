@@ -1,0 +1,79 @@
+"""Host batches go through a ring of pinned slots, chunk by chunk: the sizes where the way through it changes, with the
+caller's planes in ordinary and in pinned memory, against the oracle."""
+import numpy as np
+import pytest
+
+from cubit_b200 import MIX_FAMILY, MIX_ZIPF, Codec, build_cubin
+from cubit_b200._results import ResultPool
+
+
+def pinned_copy(a):
+    import torch
+    held = torch.empty(a.nbytes, dtype=torch.uint8, pin_memory=True).numpy().view(a.dtype).reshape(a.shape)
+    held[...] = a
+    return held
+
+
+# One chunk / several chunks the kernel reads over the bus / the first size that is copied to the device / several slots of it.
+@pytest.mark.gpu
+@pytest.mark.parametrize("pinned", [False, True])
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 16384, 16385, 65537, 262143, 262144, 262145, 1100007])
+def test_every_way_through_the_ring(codec, oracle, n, pinned):
+    place = pinned_copy if pinned else (lambda a: a)
+    words = place(oracle.synth(MIX_ZIPF, n, n, noise_ppm=20000, records=False, threads=8))
+    want = oracle.decode_batch(words, threads=8)
+    got = codec.decode_batch(words)
+    for g, w in zip(got, want):
+        assert (g == w).all()
+    assert got[3]["n_rejected"] == int((want[0] == 0xFFFF).sum()) and got[3]["n_tie"] == int(((want[2] >> 28) & 1).sum())
+    assert got[3]["n_decoded"] == n - got[3]["n_rejected"]
+    assert (codec.encode_batch(*(place(a) for a in want)) == oracle.encode_batch(*want, threads=8)).all()
+    status, counts = codec.roundtrip_batch(words)
+    assert (status == oracle.roundtrip_batch(words, threads=8)).all()
+    assert [counts["n_exact"], counts["n_mismatch"], counts["n_rejected"]] == np.bincount(status, minlength=3).tolist()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [[1], [7, 1, 300], [300000, 5, 90000]])
+def test_sections_of_a_cubin_are_gathered(codec, oracle, sizes):
+    words = oracle.synth(MIX_FAMILY, 3, sum(sizes), records=False, threads=8)
+    at = np.cumsum([0] + sizes)
+    image = build_cubin([(f"k{k}", words[at[k]:at[k + 1]].tobytes()) for k in range(len(sizes))])
+    sections, start, form, slots, ctrl, raw, counts = codec.decode_elf(image)
+    for k, (_, offset, size) in enumerate(sections):
+        here = slice(int(start[k]), int(start[k + 1]))
+        assert (raw[here].reshape(-1) == np.frombuffer(image, np.uint8)[offset:offset + size // 16 * 16]).all()
+    for g, w in zip((form, slots, ctrl), oracle.decode_batch(raw, threads=8)):
+        assert (g == w).all()
+    assert counts["n_decoded"] + counts["n_rejected"] == len(form)
+
+
+def test_result_memory_is_used_again_only_when_let_go():
+    pool = ResultPool(limit=64 << 20)
+    first = pool.empty((8, 1 << 18), np.uint32)
+    address, view = first.ctypes.data, first[3, ::7]
+    del first
+    other = pool.empty((8, 1 << 18), np.uint32)
+    assert other.ctypes.data != address                                    # a view still looks at the first
+    del view
+    again = pool.empty((8, (1 << 18) - 77), np.uint32)                     # a little smaller: fits
+    assert again.ctypes.data == address and again.shape == (8, (1 << 18) - 77)
+    assert pool.empty(100, np.uint8).base is None                          # small arrays are numpy's own
+    held = [pool.empty(20 << 20, np.uint8) for _ in range(5)]
+    del held, again, other
+    assert sum(m.nbytes for m in pool._free) <= pool.limit
+    keep = pool.empty(20 << 20, np.uint8)
+    keep[:] = 7
+    pool.clear()
+    assert not pool._free and (keep == 7).all()
+    del keep
+    assert not pool._free
+
+
+def test_results_outlive_their_codec():
+    codec = Codec(devices=())
+    a = codec._results.empty(2 << 20, np.uint8)
+    a[:] = 5
+    codec.close()
+    del codec
+    assert (a == 5).all()
