@@ -15,8 +15,8 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "_lib"
 LIB = LIB_DIR / "libcubit_b200.so"
-SOURCES = ["capi.cu", "text_api.cpp", "isa_table.cpp", "flat_table.cpp", "elf_text.cpp", "sass_text.cpp", "sass_print.cpp"]
-HEADERS = ["codec_core.cuh", "context.hpp", "work_pool.hpp", "flat_table.hpp", "isa_table.hpp", "elf_text.hpp", "sass_text.hpp", "json.hpp",
+SOURCES = ["capi.cu", "text_api.cpp", "isa_table.cpp", "flat_table.cpp", "decision_lists.cpp", "elf_text.cpp", "sass_text.cpp", "sass_print.cpp"]
+HEADERS = ["codec_core.cuh", "context.hpp", "work_pool.hpp", "flat_table.hpp", "decision_lists.hpp", "isa_table.hpp", "elf_text.hpp", "sass_text.hpp", "json.hpp",
            "../../include/cubit_b200.h"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 

@@ -26,6 +26,7 @@
 
 #include "codec_core.cuh"
 #include "context.hpp"
+#include "decision_lists.hpp"
 
 using namespace cubit;
 
@@ -42,16 +43,16 @@ enum { CNT_DECODED = 0, CNT_REJECTED, CNT_TIE, CNT_EXACT, CNT_MISMATCH, CNT_WORD
 // [begin, end) for HotShared / HotSharedEnc, the roundtrip kernel's two ranges for HotSharedRT.
 template <class HOT>
 __device__ __forceinline__ void stage_table(const FlatView&, uint32_t, uint32_t) {}
-__device__ __forceinline__ void stage_range(const FlatView& t, uint32_t begin, uint32_t end) {
-    const uint4* src = reinterpret_cast<const uint4*>(t.cold + begin);
-    const uint32_t quads = (end - begin) / 4;
+__device__ __forceinline__ void stage_quads(const uint32_t* from, uint32_t words) {
+    const uint4* src = reinterpret_cast<const uint4*>(from);
+    const uint32_t quads = words / 4;
     for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x) cb_table_smem[i] = __ldg(src + i);
     __syncthreads();
 }
 template <>
-__device__ __forceinline__ void stage_table<HotShared>(const FlatView& t, uint32_t begin, uint32_t end) { stage_range(t, begin, end); }
+__device__ __forceinline__ void stage_table<HotShared>(const FlatView& t, uint32_t begin, uint32_t end) { stage_quads(t.cold + begin, end - begin); }
 template <>
-__device__ __forceinline__ void stage_table<HotSharedEnc>(const FlatView& t, uint32_t begin, uint32_t end) { stage_range(t, begin, end); }
+__device__ __forceinline__ void stage_table<HotSharedEnc>(const FlatView& t, uint32_t begin, uint32_t end) { stage_quads(t.cold + begin, end - begin); }
 template <>
 __device__ __forceinline__ void stage_table<HotSharedRT>(const FlatView& t, uint32_t, uint32_t) {
     const uint4* src = reinterpret_cast<const uint4*>(t.cold);
@@ -79,19 +80,49 @@ __device__ __forceinline__ void block_tally(const uint32_t (&mine)[N], const int
         atomicAdd(&counters[threadIdx.x], (unsigned long long)s_acc[threadIdx.x]);
 }
 
-// WIDE: the table has leaves of more than 16 classes (the SM120 table has none; its kernels leave that path out).
+// How a kernel finds a word's variant.  `Listed` walks the decision lists of the table (decision_lists.hpp), `Scan` the classes of
+// the leaf; Scan serves the tables that have no lists.  HOT says where the table is read: HotGlobal in place, anything else
+// from shared memory, where `stage` has put it.
+// Both are bound by instruction issue and the shared-memory pipe, not by HBM.  Scan takes 364 (decode) and 283 (roundtrip)
+// warp-instructions per 32 words, a good part of them for the one or two lanes of a warp that rank candidates, try broad records
+// or follow the rules; a list has none of these steps, and the roundtrip lists need no variant and no constants of it either.
+// 64 Mi Zipf words: decode 950 -> 731 us, roundtrip with 1 % noise 838 -> 540 us.
+template <class HOT>
+struct Listed {
+    static constexpr bool kStaged = !std::is_same<HOT, HotGlobal>::value;
+    ListView t;
+    const FlatView* general;   // device memory
+    __device__ __forceinline__ void stage() const { if (kStaged) stage_quads(t.cold, t.at.words); }
+    __device__ __forceinline__ void decode(const uint4& w, uint32_t* form, uint32_t slots[8], uint32_t* ctrl) const {
+        decode_word_listed<HOT, HotGlobal>(t, general, w.x, w.y, w.z, w.w, form, slots, ctrl);
+    }
+    __device__ __forceinline__ uint32_t roundtrip(const uint4& w) const {
+        return roundtrip_word_listed<HOT, HotGlobal>(t, general, w.x, w.y, w.z, w.w);
+    }
+};
+// WIDE: the table has leaves of more than 16 classes; kernels for tables without them leave that path out.
+template <class HOT, bool WIDE>
+struct Scan {
+    static constexpr bool kStaged = !std::is_same<HOT, HotGlobal>::value;
+    FlatView t;
+    __device__ __forceinline__ void stage() const { stage_table<HOT>(t, 0, t.at.hot_words); }
+    __device__ __forceinline__ void decode(const uint4& w, uint32_t* form, uint32_t slots[8], uint32_t* ctrl) const {
+        decode_word<HOT, WIDE>(t, w.x, w.y, w.z, w.w, form, slots, ctrl);
+    }
+    __device__ __forceinline__ uint32_t roundtrip(const uint4& w) const { return roundtrip_word<HOT, WIDE>(t, w.x, w.y, w.z, w.w); }
+};
+
 // COUNT: the caller wants the counters (launches without them leave the per-word tallies out).
 // IDX is the type of the word index: uint32_t when the batch allows it (then every plane
 // address is one 32 x 32 + 64 bit multiply-add from a plane base that is the same for the
 // whole grid), uint64_t otherwise.  The next word of a thread is loaded before the current one
 // is decoded, so its latency hides behind the table walk.
-template <class HOT, class IDX, bool WIDE, bool COUNT>
-__global__ void __launch_bounds__(std::is_same<HOT, HotGlobal>::value ? kBlock : kBlockShared, 1)
-decode_kernel(FlatView tg, const uint4* __restrict__ words, uint64_t n64, uint16_t* __restrict__ form,
+template <class ENGINE, class IDX, bool COUNT>
+__global__ void __launch_bounds__(ENGINE::kStaged ? kBlockShared : kBlock, 1)
+decode_kernel(const __grid_constant__ ENGINE engine, const uint4* __restrict__ words, uint64_t n64, uint16_t* __restrict__ form,
               uint32_t* __restrict__ slots, uint64_t slot_stride, uint32_t* __restrict__ ctrl,
               unsigned long long* counters) {
-    stage_table<HOT>(tg, 0, tg.at.hot_words);
-    const FlatView& t = tg;
+    engine.stage();
     uint32_t n_ok = 0, n_tie = 0;
     const IDX n = (IDX)n64;
     const IDX step = (IDX)gridDim.x * (IDX)blockDim.x;
@@ -102,7 +133,7 @@ decode_kernel(FlatView tg, const uint4* __restrict__ words, uint64_t n64, uint16
         uint4 next = w;
         if (n - i > step) next = __ldcs(words + (i + step));
         uint32_t f, c, s[8];
-        decode_word<HOT, WIDE>(t, w.x, w.y, w.z, w.w, &f, s, &c);
+        engine.decode(w, &f, s, &c);
         __stcs(form + i, (uint16_t)f);
 #pragma unroll
         for (int k = 0; k < 8; ++k) __stcs(slots + (uint64_t)k * slot_stride + i, s[k]);
@@ -186,12 +217,11 @@ encode_kernel(FlatView tg, const uint16_t* __restrict__ form, const uint32_t* __
     }
 }
 
-template <class HOT, bool WIDE, bool COUNT>
-__global__ void __launch_bounds__(std::is_same<HOT, HotGlobal>::value ? kBlock : kBlockShared, 1)
-roundtrip_kernel(FlatView tg, const uint4* __restrict__ words, uint64_t n, uint8_t* __restrict__ status,
+template <class ENGINE, bool COUNT>
+__global__ void __launch_bounds__(ENGINE::kStaged ? kBlockShared : kBlock, 1)
+roundtrip_kernel(const __grid_constant__ ENGINE engine, const uint4* __restrict__ words, uint64_t n, uint8_t* __restrict__ status,
                  unsigned long long* counters) {
-    stage_table<HOT>(tg, 0, tg.at.hot_words);
-    const FlatView& t = tg;
+    engine.stage();
     uint32_t n_exact = 0, n_rejected = 0;
     const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -201,7 +231,7 @@ roundtrip_kernel(FlatView tg, const uint4* __restrict__ words, uint64_t n, uint8
     for (uint64_t i = first; i < n; i += step) {
         uint4 next = w;
         if (n - i > step) next = __ldcs(words + (i + step));
-        const uint32_t st = roundtrip_word<HOT, WIDE>(t, w.x, w.y, w.z, w.w);
+        const uint32_t st = engine.roundtrip(w);
         __stcs(status + i, (uint8_t)st);
         if (COUNT) { n_exact += st == RT_EXACT; n_rejected += st == RT_REJECTED; }
         w = next;
@@ -309,6 +339,10 @@ struct cubit::DeviceState {
     uint32_t hot_bytes = 0;   // decode window of the table
     uint32_t enc_bytes = 0;   // encode window
     FlatView view{};
+    // The decision lists, when the table has them; each image is staged when it fits the shared memory.
+    ListView decode_lists{}, roundtrip_lists{};
+    const FlatView* view_on_device = nullptr;
+    bool listed = false, decode_staged = false, roundtrip_staged = false;
     std::vector<void*> table_allocs;
     unsigned long long* counters = nullptr;   // kCounterSlots x CNT_WORDS
     std::vector<int> free_counter_slots;
@@ -421,9 +455,23 @@ int upload(cubit_ctx* ctx, DeviceState* d, const std::vector<T>& host, const T**
     return CUBIT_OK;
 }
 
+bool env_is_one(const char* name) {
+    const char* v = getenv(name);
+    return v && v[0] == '1';
+}
+
+// Lets the kernels of one engine use `bytes` of shared memory.
+#define CB_ENGINE(...) __VA_ARGS__
+#define CB_SMEM_LIMIT(KERNEL, bytes) CU_TRY(c, cudaFuncSetAttribute(KERNEL, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes))
+#define CB_DECODE_SMEM(ENGINE, bytes)                                                                                  \
+    CB_SMEM_LIMIT((decode_kernel<ENGINE, uint32_t, true>), bytes); CB_SMEM_LIMIT((decode_kernel<ENGINE, uint32_t, false>), bytes); \
+    CB_SMEM_LIMIT((decode_kernel<ENGINE, uint64_t, true>), bytes); CB_SMEM_LIMIT((decode_kernel<ENGINE, uint64_t, false>), bytes)
+#define CB_ROUNDTRIP_SMEM(ENGINE, bytes) \
+    CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, true>), bytes); CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, false>), bytes)
+
 // Uploads the table to one device and creates its streams and counters.  Failures report
 // through the thread-local message, as the context does not exist yet for the caller.
-int init_device(const FlatTable& ft, DeviceState* d) {
+int init_device(const FlatTable& ft, const DecisionLists& lists, DeviceState* d) {
     cubit_ctx* c = nullptr;
     CU_TRY(c, cudaSetDevice(d->device));
     CU_TRY(c, cudaDeviceGetAttribute(&d->sm_count, cudaDevAttrMultiProcessorCount, d->device));
@@ -433,37 +481,37 @@ int init_device(const FlatTable& ft, DeviceState* d) {
     d->view.cold = blob; d->view.at = ft.at;
     d->hot_bytes = ft.at.hot_words * 4;
     d->wide_leaves = ft.max_leaf_classes > 16;
-    {
-        const char* wide = getenv("CUBIT_WIDE_INDEX");
-        d->wide_index = wide && wide[0] == '1';
-    }
+    d->wide_index = env_is_one("CUBIT_WIDE_INDEX");
     d->enc_bytes = (ft.at.enc_end - ft.at.enc) * 4;
     int optin = 0;
     CU_TRY(c, cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, d->device));
     d->shared_ok = (int)d->hot_bytes + 1024 <= optin && (int)d->enc_bytes + 1024 <= optin;
     if (d->shared_ok) {
         const int hot = (int)d->hot_bytes;
-#define CB_DECODE_SMEM(IDX, WIDE, COUNT) \
-        CU_TRY(c, cudaFuncSetAttribute(decode_kernel<HotShared, IDX, WIDE, COUNT>, cudaFuncAttributeMaxDynamicSharedMemorySize, hot))
-        CB_DECODE_SMEM(uint32_t, true, true); CB_DECODE_SMEM(uint32_t, true, false);
-        CB_DECODE_SMEM(uint64_t, true, true); CB_DECODE_SMEM(uint64_t, true, false);
-        CB_DECODE_SMEM(uint32_t, false, true); CB_DECODE_SMEM(uint32_t, false, false);
-        CB_DECODE_SMEM(uint64_t, false, true); CB_DECODE_SMEM(uint64_t, false, false);
-#undef CB_DECODE_SMEM
+        CB_DECODE_SMEM(CB_ENGINE(Scan<HotShared, true>), hot); CB_DECODE_SMEM(CB_ENGINE(Scan<HotShared, false>), hot);
         CU_TRY(c, cudaFuncSetAttribute(encode_kernel<HotSharedEnc>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->enc_bytes));
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotShared, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, hot));
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotShared, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, hot));
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotShared, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, hot));
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotShared, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, hot));
+        CB_ROUNDTRIP_SMEM(CB_ENGINE(Scan<HotShared, true>), hot); CB_ROUNDTRIP_SMEM(CB_ENGINE(Scan<HotShared, false>), hot);
         CU_TRY(c, cudaFuncSetAttribute(meta_kernel<HotShared>, cudaFuncAttributeMaxDynamicSharedMemorySize, hot));
     }
     d->rt_bytes = (ft.at.sel_words + (ft.at.total_words - ft.at.rt[0])) * 4;
     d->rt_shared_ok = d->shared_ok && (int)d->rt_bytes + 1024 <= optin;
     if (d->rt_shared_ok) {
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotSharedRT, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->rt_bytes));
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotSharedRT, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->rt_bytes));
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotSharedRT, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->rt_bytes));
-        CU_TRY(c, cudaFuncSetAttribute(roundtrip_kernel<HotSharedRT, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->rt_bytes));
+        CB_ROUNDTRIP_SMEM(CB_ENGINE(Scan<HotSharedRT, true>), (int)d->rt_bytes); CB_ROUNDTRIP_SMEM(CB_ENGINE(Scan<HotSharedRT, false>), (int)d->rt_bytes);
+    }
+    if (lists.worthwhile() && !env_is_one("CUBIT_NO_LISTS")) {
+        const uint32_t *decode = nullptr, *roundtrip = nullptr;
+        int up = upload(c, d, lists.decode, &decode);
+        if (!up) up = upload(c, d, lists.roundtrip, &roundtrip);
+        if (!up) up = upload(c, d, std::vector<FlatView>(1, d->view), &d->view_on_device);
+        if (up) return up;
+        d->decode_lists = ListView{decode, lists.decode_at};
+        d->roundtrip_lists = ListView{roundtrip, lists.roundtrip_at};
+        d->listed = true;
+        const int decode_bytes = (int)lists.decode_at.words * 4, roundtrip_bytes = (int)lists.roundtrip_at.words * 4;
+        d->decode_staged = decode_bytes + 1024 <= optin;
+        d->roundtrip_staged = roundtrip_bytes + 1024 <= optin;
+        if (d->decode_staged) { CB_DECODE_SMEM(CB_ENGINE(Listed<HotShared>), decode_bytes); }
+        if (d->roundtrip_staged) { CB_ROUNDTRIP_SMEM(CB_ENGINE(Listed<HotShared>), roundtrip_bytes); }
     }
     CU_TRY(c, cudaMalloc((void**)&d->counters, sizeof(unsigned long long) * CNT_WORDS * kCounterSlots));
     for (int s = 0; s < kCounterSlots; ++s) d->free_counter_slots.push_back(s);
@@ -485,27 +533,28 @@ int grid_shared(const DeviceState* d, uint64_t n) {
     return (int)std::max<uint64_t>(1, std::min<uint64_t>((n + kBlockShared - 1) / kBlockShared, (uint64_t)d->sm_count));
 }
 
+template <class ENGINE>
+void launch_decode_with(const DeviceState* d, const ENGINE& engine, uint32_t smem, cudaStream_t s, const uint4* words, uint64_t n,
+                        uint16_t* form, uint32_t* slots, uint64_t stride, uint32_t* ctrl, unsigned long long* dc) {
+    // 32-bit word indices while index + grid size cannot wrap.
+    const bool narrow = n < (1ull << 31) && !d->wide_index;
+    const int grid = ENGINE::kStaged ? grid_shared(d, n) : grid_for(d, n), block = ENGINE::kStaged ? kBlockShared : kBlock;
+    const auto go = [&](auto kernel) { kernel<<<grid, block, smem, s>>>(engine, words, n, form, slots, stride, ctrl, dc); };
+    if (narrow) { if (dc) go(decode_kernel<ENGINE, uint32_t, true>); else go(decode_kernel<ENGINE, uint32_t, false>); }
+    else { if (dc) go(decode_kernel<ENGINE, uint64_t, true>); else go(decode_kernel<ENGINE, uint64_t, false>); }
+}
 void launch_decode(const DeviceState* d, cudaStream_t s, const uint4* words, uint64_t n, uint16_t* form, uint32_t* slots,
                    uint64_t stride, uint32_t* ctrl, unsigned long long* dc) {
-    // 32-bit word indices while index + grid size cannot wrap; kernels without the wide-leaf path when the
-    // table has no such leaf.
-    const bool narrow = n < (1ull << 31) && !d->wide_index;
-    const bool staged = use_shared(d, n);
-    const int grid = staged ? grid_shared(d, n) : grid_for(d, n), block = staged ? kBlockShared : kBlock;
-    const size_t smem = staged ? d->hot_bytes : 0;
-#define CB_LAUNCH_DECODE(HOT, IDX, WIDE)                                                                             \
-    do {                                                                                                             \
-        if (dc) decode_kernel<HOT, IDX, WIDE, true><<<grid, block, smem, s>>>(d->view, words, n, form, slots, stride, ctrl, dc); \
-        else decode_kernel<HOT, IDX, WIDE, false><<<grid, block, smem, s>>>(d->view, words, n, form, slots, stride, ctrl, dc);  \
-    } while (0)
-    if (staged) {
-        if (d->wide_leaves) { if (narrow) CB_LAUNCH_DECODE(HotShared, uint32_t, true); else CB_LAUNCH_DECODE(HotShared, uint64_t, true); }
-        else { if (narrow) CB_LAUNCH_DECODE(HotShared, uint32_t, false); else CB_LAUNCH_DECODE(HotShared, uint64_t, false); }
+    const auto go = [&](auto engine, uint32_t smem) { launch_decode_with(d, engine, smem, s, words, n, form, slots, stride, ctrl, dc); };
+    const bool large = n >= kSharedMinWords;
+    if (d->listed) {
+        if (large && d->decode_staged) go(Listed<HotShared>{d->decode_lists, d->view_on_device}, d->decode_lists.at.words * 4);
+        else go(Listed<HotGlobal>{d->decode_lists, d->view_on_device}, 0);
+    } else if (large && d->shared_ok) {
+        if (d->wide_leaves) go(Scan<HotShared, true>{d->view}, d->hot_bytes); else go(Scan<HotShared, false>{d->view}, d->hot_bytes);
     } else {
-        if (d->wide_leaves) { if (narrow) CB_LAUNCH_DECODE(HotGlobal, uint32_t, true); else CB_LAUNCH_DECODE(HotGlobal, uint64_t, true); }
-        else { if (narrow) CB_LAUNCH_DECODE(HotGlobal, uint32_t, false); else CB_LAUNCH_DECODE(HotGlobal, uint64_t, false); }
+        if (d->wide_leaves) go(Scan<HotGlobal, true>{d->view}, 0); else go(Scan<HotGlobal, false>{d->view}, 0);
     }
-#undef CB_LAUNCH_DECODE
 }
 void launch_encode(const DeviceState* d, cudaStream_t s, const uint16_t* form, const uint32_t* slots, uint64_t stride,
                    const uint32_t* ctrl, uint64_t n, uint4* words) {
@@ -519,20 +568,23 @@ void launch_encode(const DeviceState* d, cudaStream_t s, const uint16_t* form, c
 }
 void launch_roundtrip(const DeviceState* d, cudaStream_t s, const uint4* words, uint64_t n, uint8_t* status,
                       unsigned long long* dc) {
-#define CB_LAUNCH_RT(HOT, grid, block, smem)                                                          \
-    do {                                                                                              \
-        if (d->wide_leaves) {                                                                         \
-            if (dc) roundtrip_kernel<HOT, true, true><<<grid, block, smem, s>>>(d->view, words, n, status, dc);   \
-            else roundtrip_kernel<HOT, true, false><<<grid, block, smem, s>>>(d->view, words, n, status, dc);     \
-        } else {                                                                                      \
-            if (dc) roundtrip_kernel<HOT, false, true><<<grid, block, smem, s>>>(d->view, words, n, status, dc);  \
-            else roundtrip_kernel<HOT, false, false><<<grid, block, smem, s>>>(d->view, words, n, status, dc);    \
-        }                                                                                             \
-    } while (0)
-    if (use_shared(d, n) && d->rt_shared_ok) CB_LAUNCH_RT(HotSharedRT, grid_shared(d, n), kBlockShared, d->rt_bytes);
-    else if (use_shared(d, n)) CB_LAUNCH_RT(HotShared, grid_shared(d, n), kBlockShared, d->hot_bytes);
-    else CB_LAUNCH_RT(HotGlobal, grid_for(d, n), kBlock, 0);
-#undef CB_LAUNCH_RT
+    const auto go = [&](auto engine, uint32_t smem) {
+        typedef decltype(engine) ENGINE;
+        const int grid = ENGINE::kStaged ? grid_shared(d, n) : grid_for(d, n), block = ENGINE::kStaged ? kBlockShared : kBlock;
+        if (dc) roundtrip_kernel<ENGINE, true><<<grid, block, smem, s>>>(engine, words, n, status, dc);
+        else roundtrip_kernel<ENGINE, false><<<grid, block, smem, s>>>(engine, words, n, status, dc);
+    };
+    const bool large = n >= kSharedMinWords;
+    if (d->listed) {
+        if (large && d->roundtrip_staged) go(Listed<HotShared>{d->roundtrip_lists, d->view_on_device}, d->roundtrip_lists.at.words * 4);
+        else go(Listed<HotGlobal>{d->roundtrip_lists, d->view_on_device}, 0);
+    } else if (large && d->rt_shared_ok) {
+        if (d->wide_leaves) go(Scan<HotSharedRT, true>{d->view}, d->rt_bytes); else go(Scan<HotSharedRT, false>{d->view}, d->rt_bytes);
+    } else if (large && d->shared_ok) {
+        if (d->wide_leaves) go(Scan<HotShared, true>{d->view}, d->hot_bytes); else go(Scan<HotShared, false>{d->view}, d->hot_bytes);
+    } else {
+        if (d->wide_leaves) go(Scan<HotGlobal, true>{d->view}, 0); else go(Scan<HotGlobal, false>{d->view}, 0);
+    }
 }
 
 DeviceState* device_of_pointer(cubit_ctx* ctx, const void* p) {
@@ -951,6 +1003,7 @@ extern "C" int cubit_ctx_create(const char* table_path, const int* devices, int 
     if (!out || n_devices < 0 || (n_devices > 0 && !devices)) return fail(nullptr, CUBIT_ERR_INVALID, "bad argument");
     *out = nullptr;
     std::unique_ptr<cubit_ctx> ctx(new cubit_ctx);
+    DecisionLists lists;
     std::string path;
     const char* env = getenv("CUBIT_TABLE");
     if (env && *env) path = env;
@@ -959,6 +1012,7 @@ extern "C" int cubit_ctx_create(const char* table_path, const int* devices, int 
     try {
         ctx->table = IsaTable::from_file(path);
         ctx->flat = FlatTable::compile(ctx->table);
+        if (n_devices > 0) lists = DecisionLists::compile(ctx->flat);
     } catch (const std::exception& e) {
         return fail(nullptr, CUBIT_ERR_TABLE, std::string("table ") + path + ": " + e.what());
     }
@@ -977,7 +1031,7 @@ extern "C" int cubit_ctx_create(const char* table_path, const int* devices, int 
     for (int k = 0; k < n_devices; ++k) {
         std::unique_ptr<DeviceState> d(new DeviceState);
         d->device = devices[k];
-        const int rc = init_device(ft, d.get());
+        const int rc = init_device(ft, lists, d.get());
         if (rc) {   // give back what this and the earlier devices already hold
             release_device(d.get());
             for (auto& made : ctx->devs) release_device(made.get());

@@ -1,0 +1,92 @@
+"""The decision lists (csrc/decision_lists.cpp) against select_variant over the same table, word by word on the CPU: every
+entry's edge, the adversarial words, the streams, and random tables with wide leaves, ties, overlapping fields and fields
+above bit 96.  select_variant itself is compared with the oracle elsewhere; the GPU parity tests run both kinds of kernel."""
+import ctypes as C
+import json
+import subprocess
+
+import numpy as np
+import pytest
+
+import cubit_b200
+from cubit_b200 import MIX_FAMILY, MIX_UNIFORM, MIX_ZIPF
+from test_gpu_parity import adversarial_words
+from test_random_tables import random_table, table_words
+
+HERE = cubit_b200.build.PKG.parent / "tests" / "hostmirror"
+SO = HERE / "_build" / "liblists.so"
+CSRC = cubit_b200.build.CSRC
+
+
+class Lists:
+    def __init__(self, lib, text):
+        self.lib = lib
+        self.h = C.c_void_p(lib.lst_load(text, C.c_uint64(len(text))))
+        assert self.h
+        info = (C.c_uint32 * 8)()
+        lib.lst_info(self.h, info)
+        self.decode_entries, self.roundtrip_entries, self.longest, self.decode_bytes, self.roundtrip_bytes, self.runs, self.general, self.used = info
+
+    def edges(self, per_entry):
+        """Words that reach each entry and pass its test, and words that fail it in one bit."""
+        words = np.zeros((2 * per_entry * 12 * (self.decode_entries + self.roundtrip_entries), 16), np.uint8)
+        n = self.lib.lst_edges(self.h, C.c_uint64(5), per_entry, C.c_void_p(words.ctypes.data), C.c_uint64(len(words)))
+        return words[:n].copy()
+
+    def check(self, words):
+        words = np.ascontiguousarray(words)
+        first = C.c_uint64(0)
+        bad = self.lib.lst_compare(self.h, C.c_void_p(words.ctypes.data), C.c_uint64(len(words)), C.byref(first))
+        assert bad == 0, f"{bad} of {len(words)} words differ, first {words[first.value].view(np.uint64)}"
+
+
+@pytest.fixture(scope="module")
+def lists_lib():
+    srcs = [HERE / "lists.cpp"] + [CSRC / s for s in ("isa_table.cpp", "flat_table.cpp", "decision_lists.cpp")]
+    deps = srcs + [CSRC / "codec_core.cuh", CSRC / "decision_lists.hpp"]
+    if not SO.exists() or any(d.stat().st_mtime > SO.stat().st_mtime for d in deps):
+        SO.parent.mkdir(exist_ok=True)
+        subprocess.run(["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-pthread", "-Wno-unknown-pragmas", "-o", str(SO)]
+                       + [str(s) for s in srcs], check=True)
+    lib = C.CDLL(str(SO))
+    lib.lst_load.restype = C.c_void_p
+    lib.lst_compare.restype = lib.lst_edges.restype = C.c_uint64
+    return lib
+
+
+def test_lists_equal_select_variant(lists_lib, oracle):
+    lists = Lists(lists_lib, (cubit_b200.build.PKG / "tables" / "sm120.json").read_bytes())
+    assert lists.used
+    assert max(lists.decode_bytes, lists.roundtrip_bytes) + 1024 <= 227 * 1024      # staged in shared memory
+    edges = lists.edges(30)
+    assert len(edges) > 30 * lists.decode_entries
+    lists.check(edges)
+    lists.check(adversarial_words(np.random.default_rng(21), 40))
+    for mix, seed, noise in ((MIX_UNIFORM, 0, 0), (MIX_ZIPF, 7, 10000), (MIX_FAMILY, 3, 5000), (MIX_UNIFORM, 5, 500000)):
+        words = oracle.synth(mix, seed, 200000, noise_ppm=noise, threads=8, records=False).copy()
+        lists.check(words)
+        words[::2, 12:16] ^= np.random.default_rng(seed).integers(0, 256, size=(len(words[::2]), 4), dtype=np.uint8)
+        lists.check(words)                                                          # upper limbs of every kind
+
+
+@pytest.mark.parametrize("seed,n_keys,opcodes", [(s, 120, (0x210, 0x947, 0x981)) for s in range(6)] + [(7, 60, tuple(range(0x200, 0x230))),
+                                                 (8, 300, tuple(range(0x200, 0x300, 3))), (43, 275, (0x210, 0x947))])
+def test_lists_of_random_tables(lists_lib, seed, n_keys, opcodes):
+    table = random_table(seed, n_keys=n_keys, opcodes=opcodes)
+    lists = Lists(lists_lib, json.dumps(table).encode())
+    lists.check(table_words(table, np.random.default_rng(300 + seed), 60))
+    lists.check(lists.edges(20))
+    lists_lib.lst_free(lists.h)
+
+
+@pytest.mark.gpu
+def test_class_scan_kernels_match_the_lists(codec, monkeypatch):
+    """CUBIT_NO_LISTS=1 selects the kernels of tables without lists; both kinds say the same, staged and not."""
+    monkeypatch.setenv("CUBIT_NO_LISTS", "1")
+    scan = cubit_b200.Codec(devices=(0,))
+    for n in (1, 33, 5000, (1 << 19) + 77):
+        words = codec.synth(MIX_UNIFORM, 11, n, noise_ppm=30000)[0]
+        for a, b in zip(codec.decode_batch(words)[:3], scan.decode_batch(words)[:3]):
+            assert (a == b).all()
+        assert (codec.roundtrip_batch(words)[0] == scan.roundtrip_batch(words)[0]).all()
+    scan.close()
