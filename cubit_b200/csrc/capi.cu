@@ -526,8 +526,8 @@ int init_device(const FlatTable& ft, const DecisionLists& lists, DeviceState* d)
         if (!up) up = upload(c, d, lists.roundtrip, &roundtrip);
         if (!up) up = upload(c, d, std::vector<FlatView>(1, d->view), &d->view_on_device);
         if (up) return up;
-        d->decode_lists = ListView{decode, lists.decode_at};
-        d->roundtrip_lists = ListView{roundtrip, lists.roundtrip_at};
+        d->decode_lists = ListView{decode, lists.decode_at, ft.at.zero_ext};
+        d->roundtrip_lists = ListView{roundtrip, lists.roundtrip_at, ft.at.zero_ext};
         d->listed = true;
         const int decode_bytes = (int)lists.decode_at.words * 4, roundtrip_bytes = (int)lists.roundtrip_at.words * 4;
         d->decode_staged = decode_bytes + 1024 <= optin;

@@ -249,7 +249,8 @@ struct BlobLayout {
 //
 // The same lookup with the decision inside a leaf unrolled into tests in a fixed order (decision_lists.hpp): a leaf is a run
 // of entries {mask, value, outcome}, the first that agrees with the word holds the answer, and the last of every run agrees
-// with all words.  An image holds the directory, the hash nodes and their children as above (a leaf ref names the
+// with all words; where that last entry would only say that no
+// variant matches (decode) or give a status (roundtrip), the one before it says so itself (LE_STOP).  An image holds the directory, the hash nodes and their children as above (a leaf ref names the
 // first entry of its run) and the entries in planes:
 //   decode      [0] {mask[0], mask[1], mask[2], value[0]}   [1] {value[1], value[2]}   then the extraction records
 //   roundtrip   [0] {mask[0..3]}   [1] {value[0..3]}; limb 3 is the word's upper limb
@@ -263,7 +264,10 @@ enum : uint32_t {
     LE_GENERAL = 0xFFDu,        // ... select_variant has to decide
     LE_EXT = 0x3FFu,            // decode, value[0] bits 9:0: extraction record index
     LE_TIE_POS = 10,            // decode, value[0]: the tie bit of ctrl
-                                // roundtrip, mask[0] bits 11:0: the status, or LE_GENERAL
+    LE_STOP = 1u << 11,         // value[0]: the run ends here; words that fail this test match no variant (decode) or have the
+                                // other status (roundtrip)
+    LE_ELSE_POS = 2,            // roundtrip, mask[0]: the status in bits 1:0, the other status in bits 3:2 ...
+    LE_STATUS_GENERAL = 1u << 4,   // ... or select_variant has to decide
 };
 // Refs of an image are scaled by the words of what they name, which shifts their flags out of a u32.
 enum : uint32_t { LR_LEAF = 1u << 31, LR_WIDE = 1u << 30 };   // the rest: first entry of the run, or node index
@@ -274,6 +278,7 @@ struct ListLayout {
 struct ListView {
     const uint32_t* cold;       // start of the image
     ListLayout at;
+    uint32_t zero_ext;          // the extraction record of rejected words (BlobLayout)
 };
 
 struct FlatView {
@@ -1102,13 +1107,15 @@ CB_HD void decode_word_listed(const ListView& t, const FlatView* general, uint32
     const uint32_t run = find_run<HOT>(t, w0, w1, w2);
     typename HOT::Cursor p0 = HOT::at(t, t.at.entries[0] + run * 4u), p1 = HOT::at(t, t.at.entries[1] + run * 2u);
     uint32_t tag0, tag1, miss;
+#pragma unroll 1
     do {
         const Quad a = HOT::q_at(p0);
         const Pair b = HOT::d_at(p1);
         p0 = HOT::step(p0, 4u); p1 = HOT::step(p1, 2u);
         miss = ((w0 ^ a.w) & a.x & LE_TEST0) | ((w1 ^ b.x) & a.y) | ((w2 ^ b.y) & a.z);
         tag0 = a.x; tag1 = a.w;
-    } while (miss);
+    } while (miss && !(tag1 & LE_STOP));
+    if (miss) { tag0 = LE_NO_VARIANT; tag1 = t.zero_ext; }
     uint32_t variant = tag0 & LE_OUTCOME, ext = tag1 & LE_EXT;
     uint32_t c = ctrl_from_raw(w0, w3) | ((tag1 << (28 - LE_TIE_POS)) & (1u << 28));
     if (variant == LE_GENERAL) {
@@ -1134,15 +1141,16 @@ template <class HOT, class GENERAL>
 CB_HD uint32_t roundtrip_word_listed(const ListView& t, const FlatView* general, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {
     const uint32_t run = find_run<HOT>(t, w0, w1, w2);
     typename HOT::Cursor p0 = HOT::at(t, t.at.entries[0] + run * 4u), p1 = HOT::at(t, t.at.entries[1] + run * 4u);
-    uint32_t tag, miss;
+    uint32_t tag, miss, stop;
+#pragma unroll 1
     do {
         const Quad m = HOT::q_at(p0), v = HOT::q_at(p1);
         p0 = HOT::step(p0, 4u); p1 = HOT::step(p1, 4u);
         miss = ((w0 ^ v.x) & m.x & LE_TEST0) | ((w1 ^ v.y) & m.y) | ((w2 ^ v.z) & m.z) | ((w3 ^ v.w) & m.w);
-        tag = m.x;
-    } while (miss);
-    const uint32_t status = tag & LE_OUTCOME;
-    return status == LE_GENERAL ? roundtrip_general<GENERAL>(general, w0, w1, w2, w3) : status;
+        tag = m.x; stop = v.x & LE_STOP;
+    } while (miss && !stop);
+    if (tag & LE_STATUS_GENERAL) return roundtrip_general<GENERAL>(general, w0, w1, w2, w3);
+    return (miss ? tag >> LE_ELSE_POS : tag) & 3u;
 }
 
 // ---- kernel metadata -------------------------------------------------------------------

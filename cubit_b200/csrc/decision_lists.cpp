@@ -77,7 +77,7 @@ void tidy(List* list) {
 }
 
 // An outcome: a variant (FORM_NONE: none matches) | tie << 16, or a status, or one of these.
-constexpr uint32_t kGeneral = 0x80000000u, kNoOpcode = 0x40000000u;
+constexpr uint32_t kGeneral = 0x80000000u, kNoOpcode = 0x40000000u, kNone = 0xFFFFFFFFu;
 // Two candidates whose popcounts differ in more open bits than this are left to select_variant: every bit that has to be
 // asked nearly doubles the list (four bits make 10 entries of one, eight 78 and more).
 constexpr int kOpenBits = 4;
@@ -309,7 +309,9 @@ struct LeafDecision {
 struct ImageBuilder {
     const FlatTable& ft;
     const bool roundtrip;
-    std::vector<List> runs;
+    // A run as it is stored: its entries, and what words get that pass none of them (kNone: the last entry takes every word).
+    struct Run { List list; uint32_t otherwise; };
+    std::vector<Run> runs;
     std::map<std::vector<uint64_t>, uint32_t> known_runs;   // the same run is stored once
     std::map<std::pair<uint32_t, uint32_t>, uint32_t> leaf_run;   // (leaf ref, opcode bits) -> entry index
     uint32_t entries = 0, longest = 0;
@@ -323,7 +325,19 @@ struct ImageBuilder {
             flat.push_back(e.outcome);
         }
         const auto made = known_runs.emplace(flat, entries);
-        if (made.second) { runs.push_back(l); entries += uint32_t(l.size()); longest = std::max(longest, uint32_t(l.size())); }
+        if (made.second) {
+            Run r{l, kNone};
+            // The test before a last entry can say what that entry would: not when it sends its own words to select_variant
+            // (they are told apart by the outcome alone).
+            const uint32_t last = l.back().outcome;
+            if (l.size() > 1 && l[l.size() - 2].outcome != kGeneral && (roundtrip ? last != kGeneral : last == FORM_NONE)) {
+                r.otherwise = last;
+                r.list.pop_back();
+            }
+            entries += uint32_t(r.list.size());
+            longest = std::max(longest, uint32_t(r.list.size()));
+            runs.push_back(std::move(r));
+        }
         return made.first->second;
     }
     uint32_t leaf(uint32_t ref, uint32_t opcode) {
@@ -353,12 +367,16 @@ struct ImageBuilder {
         for (uint32_t op = 0; op < 4096; ++op)
             if (const uint32_t ref = ft.blob[ft.at.dir + op]) dir[op] = convert(ref, op, &children);
         std::vector<uint32_t> plane[2], nodes[2];
-        for (const List& l : runs)
-            for (const Entry& e : l) {
+        for (const Run& r : runs)
+            for (size_t i = 0; i < r.list.size(); ++i) {
+                const Entry& e = r.list[i];
+                const bool stop = r.otherwise != kNone && i + 1 == r.list.size();
                 uint32_t m[4], v[4];
                 for (int k = 0; k < 4; ++k) { m[k] = uint32_t(e.test.mask >> (32 * k)); v[k] = uint32_t(e.test.value >> (32 * k)); }
+                if (stop) v[0] |= LE_STOP;
                 if (roundtrip) {
-                    m[0] |= e.outcome == kGeneral ? (uint32_t)LE_GENERAL : e.outcome;
+                    m[0] |= e.outcome == kGeneral ? (uint32_t)LE_STATUS_GENERAL : e.outcome;
+                    if (stop) m[0] |= r.otherwise << LE_ELSE_POS;
                     plane[0].insert(plane[0].end(), m, m + 4);
                     plane[1].insert(plane[1].end(), v, v + 4);
                     continue;
@@ -408,8 +426,8 @@ DecisionLists DecisionLists::compile(const FlatTable& ft) {
         (which ? d.roundtrip_entries : d.decode_entries) = b.entries;
         if (which == 0) {
             d.runs = uint32_t(b.runs.size());
-            for (const List& l : b.runs)
-                d.general_runs += std::any_of(l.begin(), l.end(), [](const Entry& e) { return e.outcome == kGeneral; }) ? 1 : 0;
+            for (const auto& r : b.runs)
+                d.general_runs += std::any_of(r.list.begin(), r.list.end(), [](const Entry& e) { return e.outcome == kGeneral; }) ? 1 : 0;
         }
         d.longest = std::max(d.longest, b.longest);
     }

@@ -26,8 +26,8 @@ void* lst_load(const char* text, uint64_t len) {
         l->flat = FlatTable::compile(l->table);
         l->lists = DecisionLists::compile(l->flat);
         l->general = FlatView{l->flat.blob.data(), l->flat.at};
-        l->decode = ListView{l->lists.decode.data(), l->lists.decode_at};
-        l->roundtrip = ListView{l->lists.roundtrip.data(), l->lists.roundtrip_at};
+        l->decode = ListView{l->lists.decode.data(), l->lists.decode_at, l->flat.at.zero_ext};
+        l->roundtrip = ListView{l->lists.roundtrip.data(), l->lists.roundtrip_at, l->flat.at.zero_ext};
         return l;
     } catch (const std::exception&) { return nullptr; }
 }
@@ -83,6 +83,7 @@ uint64_t lst_edges(void* h, uint64_t seed, uint32_t per_entry, uint32_t* words, 
                 const uint32_t* p1 = &img[at.entries[1] + e * (rt ? 4 : 2)];
                 if (rt) { memcpy(m, p0, 16); memcpy(v, p1, 16); }
                 else { memcpy(m, p0, 12); v[0] = p0[3]; v[1] = p1[0]; v[2] = p1[1]; }
+                const bool stop = (v[0] & LE_STOP) != 0;
                 m[0] &= LE_TEST0; v[0] &= LE_TEST0;
                 if (!(m[0] | m[1] | m[2] | m[3])) break;
                 for (uint32_t k = 0; k < per_entry && n < room; ++k, ++n) {
@@ -95,6 +96,7 @@ uint64_t lst_edges(void* h, uint64_t seed, uint32_t per_entry, uint32_t* words, 
                         w[bit >> 5] ^= 1u << (bit & 31);
                     }
                 }
+                if (stop) break;
             }
         }
     }
