@@ -103,21 +103,21 @@ __device__ __forceinline__ void block_tally(const uint32_t (&mine)[N], const int
 // How a kernel finds a word's variant.  `Listed` walks the decision lists of the table (decision_lists.hpp), `Scan` the classes of
 // the leaf; Scan serves the tables that have no lists.  HOT says where the table is read: HotGlobal in place, anything else
 // from shared memory, where `stage` has put it.
-// Both are bound by instruction issue and the shared-memory pipe, not by HBM.  Scan takes 364 (decode) and 283 (roundtrip)
-// warp-instructions per 32 words, a good part of them for the one or two lanes of a warp that rank candidates, try broad records
-// or follow the rules; a list has none of these steps, and the roundtrip lists need no variant and no constants of it either.
-// 64 Mi Zipf words: decode 950 -> 731 us, roundtrip with 1 % noise 838 -> 540 us.
+// Scan takes 364 (decode) and 283 (roundtrip) warp-instructions and 84 and 70 wavefronts of the shared-memory pipe per 32
+// words, a good part of them for the one or two lanes of a warp that rank candidates, try broad records or follow the rules.  A
+// list has none of these steps, and the roundtrip lists need no variant and no constants of it either: 223 and 152 instructions,
+// 56 and 42 wavefronts, 40 and 32 registers.  64 Mi Zipf words, with 1 % noise: decode 853 -> 666 us (then bound by the order of
+// its stores), roundtrip 687 -> 375 us (bound by the shared-memory pipe, 82 %, and the integer pipe, 69 %).
 template <class HOT>
 struct Listed {
     static constexpr bool kStaged = !std::is_same<HOT, HotGlobal>::value;
     ListView t;
-    const FlatView* general;   // device memory
     __device__ __forceinline__ void stage() const { if (kStaged) stage_quads(t.cold, t.at.words); }
     __device__ __forceinline__ void decode(const uint4& w, uint32_t* form, uint32_t slots[8], uint32_t* ctrl) const {
-        decode_word_listed<HOT, HotGlobal>(t, general, w.x, w.y, w.z, w.w, form, slots, ctrl);
+        decode_word_listed<HOT>(t, w.x, w.y, w.z, w.w, form, slots, ctrl);
     }
     __device__ __forceinline__ uint32_t roundtrip(const uint4& w) const {
-        return roundtrip_word_listed<HOT, HotGlobal>(t, general, w.x, w.y, w.z, w.w);
+        return roundtrip_word_listed<HOT>(t, w.x, w.y, w.z, w.w);
     }
 };
 // WIDE: the table has leaves of more than 16 classes; kernels for tables without them leave that path out.
@@ -237,18 +237,19 @@ encode_kernel(FlatView tg, const uint16_t* __restrict__ form, const uint32_t* __
     }
 }
 
-template <class ENGINE, bool COUNT>
+template <class ENGINE, class IDX, bool COUNT>
 __global__ void __launch_bounds__(ENGINE::kStaged ? kBlockShared : kBlock, 1)
-roundtrip_kernel(const __grid_constant__ ENGINE engine, const uint4* __restrict__ words, uint64_t n, uint8_t* __restrict__ status,
+roundtrip_kernel(const __grid_constant__ ENGINE engine, const uint4* __restrict__ words, uint64_t n64, uint8_t* __restrict__ status,
                  Tally counters) {
     engine.stage();
     uint32_t n_exact = 0, n_rejected = 0;
-    const uint64_t step = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t first = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const IDX n = (IDX)n64;
+    const IDX step = (IDX)gridDim.x * (IDX)blockDim.x;
+    const IDX first = (IDX)blockIdx.x * (IDX)blockDim.x + (IDX)threadIdx.x;
     // The next word of a thread is loaded before the current one is checked.
     uint4 w = make_uint4(0u, 0u, 0u, 0u);
     if (first < n) w = __ldcs(words + first);
-    for (uint64_t i = first; i < n; i += step) {
+    for (IDX i = first; i < n; i += step) {
         uint4 next = w;
         if (n - i > step) next = __ldcs(words + (i + step));
         const uint32_t st = engine.roundtrip(w);
@@ -361,7 +362,6 @@ struct cubit::DeviceState {
     FlatView view{};
     // The decision lists, when the table has them; each image is staged when it fits the shared memory.
     ListView decode_lists{}, roundtrip_lists{};
-    const FlatView* view_on_device = nullptr;
     bool listed = false, decode_staged = false, roundtrip_staged = false;
     std::vector<void*> table_allocs;
     CountSlot* counters = nullptr;            // kCounterSlots
@@ -489,7 +489,8 @@ bool env_is_one(const char* name) {
     CB_SMEM_LIMIT((decode_kernel<ENGINE, uint32_t, true>), bytes); CB_SMEM_LIMIT((decode_kernel<ENGINE, uint32_t, false>), bytes); \
     CB_SMEM_LIMIT((decode_kernel<ENGINE, uint64_t, true>), bytes); CB_SMEM_LIMIT((decode_kernel<ENGINE, uint64_t, false>), bytes)
 #define CB_ROUNDTRIP_SMEM(ENGINE, bytes) \
-    CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, true>), bytes); CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, false>), bytes)
+    CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, uint32_t, true>), bytes); CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, uint32_t, false>), bytes); \
+    CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, uint64_t, true>), bytes); CB_SMEM_LIMIT((roundtrip_kernel<ENGINE, uint64_t, false>), bytes)
 
 // Uploads the table to one device and creates its streams and counters.  Failures report
 // through the thread-local message, as the context does not exist yet for the caller.
@@ -520,11 +521,10 @@ int init_device(const FlatTable& ft, const DecisionLists& lists, DeviceState* d)
     if (d->rt_shared_ok) {
         CB_ROUNDTRIP_SMEM(CB_ENGINE(Scan<HotSharedRT, true>), (int)d->rt_bytes); CB_ROUNDTRIP_SMEM(CB_ENGINE(Scan<HotSharedRT, false>), (int)d->rt_bytes);
     }
-    if (lists.worthwhile() && !env_is_one("CUBIT_NO_LISTS")) {
+    if (!lists.decode.empty() && !env_is_one("CUBIT_NO_LISTS")) {
         const uint32_t *decode = nullptr, *roundtrip = nullptr;
         int up = upload(c, d, lists.decode, &decode);
         if (!up) up = upload(c, d, lists.roundtrip, &roundtrip);
-        if (!up) up = upload(c, d, std::vector<FlatView>(1, d->view), &d->view_on_device);
         if (up) return up;
         d->decode_lists = ListView{decode, lists.decode_at, ft.at.zero_ext};
         d->roundtrip_lists = ListView{roundtrip, lists.roundtrip_at, ft.at.zero_ext};
@@ -572,8 +572,8 @@ void launch_decode(const DeviceState* d, cudaStream_t s, const uint4* words, uin
     const auto go = [&](auto engine, uint32_t smem) { launch_decode_with(d, engine, smem, s, words, n, form, slots, stride, ctrl, dc); };
     const bool large = n >= kSharedMinWords;
     if (d->listed) {
-        if (large && d->decode_staged) go(Listed<HotShared>{d->decode_lists, d->view_on_device}, d->decode_lists.at.words * 4);
-        else go(Listed<HotGlobal>{d->decode_lists, d->view_on_device}, 0);
+        if (large && d->decode_staged) go(Listed<HotShared>{d->decode_lists}, d->decode_lists.at.words * 4);
+        else go(Listed<HotGlobal>{d->decode_lists}, 0);
     } else if (large && d->shared_ok) {
         if (d->wide_leaves) go(Scan<HotShared, true>{d->view}, d->hot_bytes); else go(Scan<HotShared, false>{d->view}, d->hot_bytes);
     } else {
@@ -595,13 +595,15 @@ void launch_roundtrip(const DeviceState* d, cudaStream_t s, const uint4* words, 
     const auto go = [&](auto engine, uint32_t smem) {
         typedef decltype(engine) ENGINE;
         const int grid = ENGINE::kStaged ? grid_shared(d, n) : grid_for(d, n), block = ENGINE::kStaged ? kBlockShared : kBlock;
-        if (dc.slot) roundtrip_kernel<ENGINE, true><<<grid, block, smem, s>>>(engine, words, n, status, dc);
-        else roundtrip_kernel<ENGINE, false><<<grid, block, smem, s>>>(engine, words, n, status, dc);
+        const bool narrow = n < (1ull << 31) && !d->wide_index;   // as in launch_decode_with
+        const auto run = [&](auto kernel) { kernel<<<grid, block, smem, s>>>(engine, words, n, status, dc); };
+        if (narrow) { if (dc.slot) run(roundtrip_kernel<ENGINE, uint32_t, true>); else run(roundtrip_kernel<ENGINE, uint32_t, false>); }
+        else { if (dc.slot) run(roundtrip_kernel<ENGINE, uint64_t, true>); else run(roundtrip_kernel<ENGINE, uint64_t, false>); }
     };
     const bool large = n >= kSharedMinWords;
     if (d->listed) {
-        if (large && d->roundtrip_staged) go(Listed<HotShared>{d->roundtrip_lists, d->view_on_device}, d->roundtrip_lists.at.words * 4);
-        else go(Listed<HotGlobal>{d->roundtrip_lists, d->view_on_device}, 0);
+        if (large && d->roundtrip_staged) go(Listed<HotShared>{d->roundtrip_lists}, d->roundtrip_lists.at.words * 4);
+        else go(Listed<HotGlobal>{d->roundtrip_lists}, 0);
     } else if (large && d->rt_shared_ok) {
         if (d->wide_leaves) go(Scan<HotSharedRT, true>{d->view}, d->rt_bytes); else go(Scan<HotSharedRT, false>{d->view}, d->rt_bytes);
     } else if (large && d->shared_ok) {

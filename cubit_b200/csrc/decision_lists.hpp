@@ -21,13 +21,10 @@ struct DecisionLists {
     std::vector<uint32_t> decode, roundtrip;   // table images for the kernels; offsets in `at` (ListLayout)
     ListLayout decode_at{}, roundtrip_at{};
     uint32_t decode_entries = 0, roundtrip_entries = 0, longest = 0;
-    uint32_t runs = 0, general_runs = 0;       // runs of the decode image; those of them that send some word to select_variant
 
-    // Lists pay while few words are sent to select_variant: it then runs out of line, for one or two lanes of a warp and on a
-    // table in global memory.  Tables of wide leaves keep the kernels that scan classes.
-    bool worthwhile() const { return !decode.empty() && general_runs * 16 <= runs; }
-
-    // Both images are empty when an entry has too few bits for the table's variants or field layouts.
+    // Both images are empty when a table does not fit the form: leaves of more than 16 classes, more variants or field layouts
+    // than an entry has bits for, a leaf whose decision takes hundreds of entries, ones among the constant bits of the upper limb.
+    // Such tables keep the kernels that scan classes.
     static DecisionLists compile(const FlatTable& ft);
 };
 

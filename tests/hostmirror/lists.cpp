@@ -32,12 +32,12 @@ void* lst_load(const char* text, uint64_t len) {
     } catch (const std::exception&) { return nullptr; }
 }
 void lst_free(void* h) { delete (Lists*)h; }
-// out: entries of the decode and the roundtrip image, longest run, bytes of the two images, runs, runs that send words to
-// select_variant, whether the product would use the lists
+// out: entries of the decode and the roundtrip image, longest run, bytes of the two images, balances of the decode image
 void lst_info(void* h, uint32_t* out) {
     const DecisionLists& l = ((Lists*)h)->lists;
-    const uint32_t v[8] = {l.decode_entries, l.roundtrip_entries, l.longest, (uint32_t)l.decode.size() * 4, (uint32_t)l.roundtrip.size() * 4,
-                           l.runs, l.general_runs, l.worthwhile()};
+    uint32_t balances = 0;
+    for (uint32_t e = 0; e < l.decode_entries; ++e) balances += (l.decode[l.decode_at.entries[0] + 4 * e] & LE_OUTCOME) == LE_BALANCE;
+    const uint32_t v[6] = {l.decode_entries, l.roundtrip_entries, l.longest, (uint32_t)l.decode.size() * 4, (uint32_t)l.roundtrip.size() * 4, balances};
     memcpy(out, v, sizeof v);
 }
 // Words for which the two disagree, record by record and status by status; `first_bad` names the first of them.
@@ -48,9 +48,9 @@ uint64_t lst_compare(void* h, const uint32_t* words, uint64_t n, uint64_t* first
         const uint32_t* w = words + 4 * i;
         uint32_t f[2], c[2], s[2][8];
         decode_word<HotPlain>(l->general, w[0], w[1], w[2], w[3], &f[0], s[0], &c[0]);
-        decode_word_listed<HotPlain, HotPlain>(l->decode, &l->general, w[0], w[1], w[2], w[3], &f[1], s[1], &c[1]);
+        decode_word_listed<HotPlain>(l->decode, w[0], w[1], w[2], w[3], &f[1], s[1], &c[1]);
         const uint32_t a = roundtrip_word<HotPlain>(l->general, w[0], w[1], w[2], w[3]);
-        const uint32_t b = roundtrip_word_listed<HotPlain, HotPlain>(l->roundtrip, &l->general, w[0], w[1], w[2], w[3]);
+        const uint32_t b = roundtrip_word_listed<HotPlain>(l->roundtrip, w[0], w[1], w[2], w[3]);
         if (f[0] != f[1] || c[0] != c[1] || memcmp(s[0], s[1], sizeof s[0]) || a != b) {
             if (!bad) *first_bad = i;
             ++bad;
@@ -68,36 +68,52 @@ uint64_t lst_edges(void* h, uint64_t seed, uint32_t per_entry, uint32_t* words, 
         const ListLayout& at = rt ? l->lists.roundtrip_at : l->lists.decode_at;
         // Opcode bits of a run: every directory entry that leads to it.
         std::vector<std::pair<uint32_t, uint32_t>> todo;
-        for (uint32_t op = 0; op < 4096; ++op) todo.push_back({img[at.dir + op], op});
+        const auto add_children = [&](const uint32_t* node, uint32_t shift, uint32_t op) {
+            for (uint32_t c = 0; c < (1u << (32 - shift)); ++c) todo.push_back({img[at.children + node[NR_CHILD] + c], op});
+        };
+        for (uint32_t op = 0; op < 4096; ++op) {
+            const uint32_t* d = &img[at.dir + op * 4];
+            if (!(d[NR_SHIFT] & LD_SHIFT)) todo.push_back({img[at.children + d[NR_CHILD]], op});   // no node
+            else add_children(d, d[NR_SHIFT] & LD_SHIFT, op);
+        }
         while (!todo.empty()) {
             const uint32_t ref = todo.back().first, op = todo.back().second;
             todo.pop_back();
             if (!(ref & LR_LEAF)) {
-                const uint32_t* node = &img[at.nodes[0] + (ref & 0xFFFFFu) * 4];
-                for (uint32_t c = 0; c < (1u << (32 - node[NR_SHIFT])); ++c) todo.push_back({img[at.children + node[NR_CHILD] + c], op});
+                const uint32_t* node = &img[at.nodes[0] + (ref & 0x3FFFFFFFu) * 4];
+                add_children(node, node[NR_SHIFT], op);
                 continue;
             }
-            for (uint32_t e = ref & 0xFFFFFu;; ++e) {
-                uint32_t m[4] = {0, 0, 0, 0}, v[4] = {0, 0, 0, 0};
-                const uint32_t* p0 = &img[at.entries[0] + e * 4];
-                const uint32_t* p1 = &img[at.entries[1] + e * (rt ? 4 : 2)];
-                if (rt) { memcpy(m, p0, 16); memcpy(v, p1, 16); }
-                else { memcpy(m, p0, 12); v[0] = p0[3]; v[1] = p1[0]; v[2] = p1[1]; }
-                const bool stop = (v[0] & LE_STOP) != 0;
-                m[0] &= LE_TEST0; v[0] &= LE_TEST0;
-                if (!(m[0] | m[1] | m[2] | m[3])) break;
-                for (uint32_t k = 0; k < per_entry && n < room; ++k, ++n) {
-                    uint32_t* w = words + 4 * n;
-                    for (int j = 0; j < 4; ++j) w[j] = (v[j] & m[j]) | ((uint32_t)(synth_draw(seed, n, j) >> 32) & ~m[j]);
-                    w[0] = (w[0] & ~0xFFFu) | op;
-                    if (k & 1) {   // one bit of the test the other way
-                        uint32_t bit = (uint32_t)(synth_draw(seed, n, 9) % 128);
-                        while (!((m[bit >> 5] >> (bit & 31)) & 1u)) bit = (bit + 1) % 128;
-                        w[bit >> 5] ^= 1u << (bit & 31);
+            std::vector<uint32_t> starts{ref & 0x3FFFFFFFu};   // the run, and the lists behind its balances
+            for (size_t s = 0; s < starts.size(); ++s)
+                for (uint32_t e = starts[s];; ++e) {
+                    uint32_t m[4] = {0, 0, 0, 0}, v[4] = {0, 0, 0, 0};
+                    const uint32_t* p0 = &img[at.entries[0] + e * 4];
+                    const uint32_t* p1 = &img[at.entries[1] + e * 2];
+                    memcpy(m, p0, 12);
+                    v[0] = p0[3]; v[1] = p1[0]; v[2] = p1[1];
+                    if (rt && (v[0] & LE_UPPER_REST)) m[3] = 0xE00001FFu | ((v[0] & LE_UPPER_REUSE) << 26);
+                    const bool balance = rt ? (v[0] & LE_STATUS_BALANCE) != 0 : (m[0] & LE_OUTCOME) == LE_BALANCE;
+                    if (balance) {
+                        const uint32_t record = e + 1 + (rt ? (v[0] >> LE_STATUS_POS) & LE_AHEAD_MOST : v[0] & LE_EXT);
+                        starts.push_back(record + 1);
+                        starts.push_back(record + 1 + (img[at.entries[0] + record * 4] & LB_LOW));
                     }
+                    const bool stop = (v[0] & LE_STOP) != 0;
+                    m[0] &= LE_TEST0; v[0] &= LE_TEST0;
+                    if (!(m[0] | m[1] | m[2] | m[3])) break;
+                    for (uint32_t k = 0; k < per_entry && n < room; ++k, ++n) {
+                        uint32_t* w = words + 4 * n;
+                        for (int j = 0; j < 4; ++j) w[j] = (v[j] & m[j]) | ((uint32_t)(synth_draw(seed, n, j) >> 32) & ~m[j]);
+                        w[0] = (w[0] & ~0xFFFu) | op;
+                        if (k & 1) {   // one bit of the test the other way
+                            uint32_t bit = (uint32_t)(synth_draw(seed, n, 9) % 128);
+                            while (!((m[bit >> 5] >> (bit & 31)) & 1u)) bit = (bit + 1) % 128;
+                            w[bit >> 5] ^= 1u << (bit & 31);
+                        }
+                    }
+                    if (stop) break;
                 }
-                if (stop) break;
-            }
         }
     }
     return n;
