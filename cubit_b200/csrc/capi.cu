@@ -36,17 +36,24 @@ namespace {
 
 constexpr int kBlock = 256;          // table in global memory
 constexpr int kBlockShared = 1024;   // table staged in shared memory, one CTA per SM
-constexpr uint64_t kSharedMinWords = 1u << 17;   // below this the staging copy is not worth it
+// Below these the staging copy is not worth it.  Encode: 10.3 against 12.3 us for 47,244 words, equal at 131,072.  The lists of
+// decode and roundtrip: equal at 20,000 words (10.3 us), 10.2 against 12.3 us at 100,000.
+constexpr uint64_t kSharedMinWords = 1u << 17;
+constexpr uint64_t kListedMinWords = 1u << 15;
 enum { CNT_DECODED = 0, CNT_REJECTED, CNT_TIE, CNT_EXACT, CNT_MISMATCH, CNT_WORDS };
 
 // Copies the kernel's window of the blob into dynamic shared memory, by the whole CTA: words
-// [begin, end) for HotShared / HotSharedEnc, the roundtrip kernel's two ranges for HotSharedRT.
+// [begin, end) for HotShared / HotSharedEnc, the roundtrip kernel's two ranges for HotSharedRT.  All copies of a thread are in flight
+// at once (through registers it was four at a time: roundtrip of 1,000,003 words 18.5 us, this way 16.4).
 template <class HOT>
 __device__ __forceinline__ void stage_table(const FlatView&, uint32_t, uint32_t) {}
 __device__ __forceinline__ void stage_quads(const uint32_t* from, uint32_t words) {
     const uint4* src = reinterpret_cast<const uint4*>(from);
     const uint32_t quads = words / 4;
-    for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x) cb_table_smem[i] = __ldg(src + i);
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(cb_table_smem);
+    for (uint32_t i = threadIdx.x; i < quads; i += blockDim.x)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(to + i * 16u), "l"(src + i) : "memory");
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 }
 template <>
@@ -570,7 +577,7 @@ void launch_decode_with(const DeviceState* d, const ENGINE& engine, uint32_t sme
 void launch_decode(const DeviceState* d, cudaStream_t s, const uint4* words, uint64_t n, uint16_t* form, uint32_t* slots,
                    uint64_t stride, uint32_t* ctrl, Tally dc) {
     const auto go = [&](auto engine, uint32_t smem) { launch_decode_with(d, engine, smem, s, words, n, form, slots, stride, ctrl, dc); };
-    const bool large = n >= kSharedMinWords;
+    const bool large = n >= (d->listed ? kListedMinWords : kSharedMinWords);
     if (d->listed) {
         if (large && d->decode_staged) go(Listed<HotShared>{d->decode_lists}, d->decode_lists.at.words * 4);
         else go(Listed<HotGlobal>{d->decode_lists}, 0);
@@ -600,7 +607,7 @@ void launch_roundtrip(const DeviceState* d, cudaStream_t s, const uint4* words, 
         if (narrow) { if (dc.slot) run(roundtrip_kernel<ENGINE, uint32_t, true>); else run(roundtrip_kernel<ENGINE, uint32_t, false>); }
         else { if (dc.slot) run(roundtrip_kernel<ENGINE, uint64_t, true>); else run(roundtrip_kernel<ENGINE, uint64_t, false>); }
     };
-    const bool large = n >= kSharedMinWords;
+    const bool large = n >= (d->listed ? kListedMinWords : kSharedMinWords);
     if (d->listed) {
         if (large && d->roundtrip_staged) go(Listed<HotShared>{d->roundtrip_lists}, d->roundtrip_lists.at.words * 4);
         else go(Listed<HotGlobal>{d->roundtrip_lists}, 0);
