@@ -4,9 +4,10 @@
 // consecutive 16-byte words (512 contiguous bytes) and writes 32 consecutive entries of
 // every output plane, so all global traffic is coalesced and uses streaming hints.  The
 // per-word table lookups are data dependent and diverge between lanes, so the hot part of
-// the ISA table (about 215 KB) is staged into shared memory once per CTA by persistent
-// CTAs (one per SM, 1024 threads); small batches use a variant that reads the table through
-// the read-only global path instead of paying for the staging.
+// the ISA table (about 160 KB of decision lists, or 215 KB of classes where a table has no
+// lists) is staged into shared memory once per CTA by persistent CTAs (one per SM, 1024
+// threads); small batches use a variant that reads the table through the read-only global
+// path instead of paying for the staging.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
 
@@ -112,9 +113,9 @@ __device__ __forceinline__ void block_tally(const uint32_t (&mine)[N], const int
 // from shared memory, where `stage` has put it.
 // Scan takes 364 (decode) and 283 (roundtrip) warp-instructions and 84 and 70 wavefronts of the shared-memory pipe per 32
 // words, a good part of them for the one or two lanes of a warp that rank candidates, try broad records or follow the rules.  A
-// list has none of these steps, and the roundtrip lists need no variant and no constants of it either: 223 and 152 instructions,
+// list has none of these steps, and the roundtrip lists need no variant and no constants of it either: 226 and 144 instructions,
 // 56 and 42 wavefronts, 40 and 32 registers.  64 Mi Zipf words, with 1 % noise: decode 853 -> 666 us (then bound by the order of
-// its stores), roundtrip 687 -> 375 us (bound by the shared-memory pipe, 82 %, and the integer pipe, 69 %).
+// its stores), roundtrip 687 -> 375 us (bound by the shared-memory pipe, 88 % busy).
 template <class HOT>
 struct Listed {
     static constexpr bool kStaged = !std::is_same<HOT, HotGlobal>::value;
