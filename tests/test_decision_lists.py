@@ -99,3 +99,30 @@ def test_class_scan_kernels_match_the_lists(codec, monkeypatch):
             assert (a == b).all()
         assert (codec.roundtrip_batch(words)[0] == scan.roundtrip_batch(words)[0]).all()
     scan.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 31, (1 << 15) - 1, 1 << 15, (1 << 15) + 1, 148 * 1024 + 3])
+def test_device_batches_around_the_staging_threshold(codec, oracle, n):
+    """Lists read in place below 32 Ki words, staged from there on; counted (the last block writes the sums) and not, the
+    counted call twice, so that a slot that was not left at zero would show."""
+    import torch
+    words = oracle.synth(MIX_UNIFORM, 17, n, noise_ppm=50000, threads=8, records=False)
+    form, slots, ctrl = oracle.decode_batch(words, threads=8)
+    status = oracle.roundtrip_batch(words, threads=8)
+    w = torch.from_numpy(np.ascontiguousarray(words)).cuda()
+    f = torch.zeros(n, dtype=torch.int16, device="cuda"); s = torch.zeros((8, n), dtype=torch.int32, device="cuda")
+    c = torch.zeros(n, dtype=torch.int32, device="cuda"); z = torch.full((n,), 9, dtype=torch.uint8, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    for want in (True, True, False):
+        for t in (f, s, c):
+            t.zero_()
+        counts = codec.decode_device(w.data_ptr(), n, f.data_ptr(), s.data_ptr(), c.data_ptr(), stream, want)
+        rcounts = codec.roundtrip_device(w.data_ptr(), n, z.data_ptr(), stream, want)
+        torch.cuda.synchronize()
+        assert (f.cpu().numpy().view(np.uint16) == form).all() and (s.cpu().numpy().view(np.uint32) == slots).all()
+        assert (c.cpu().numpy().view(np.uint32) == ctrl).all() and (z.cpu().numpy() == status).all()
+        if want:
+            assert counts["n_rejected"] == int((ctrl >> 30 != 0).sum()) and counts["n_decoded"] == n - counts["n_rejected"]
+            assert counts["n_tie"] == int(((ctrl >> 28) & 1).sum())
+            assert [rcounts[k] for k in ("n_exact", "n_mismatch", "n_rejected")] == np.bincount(status, minlength=3).tolist()
